@@ -288,7 +288,7 @@ void SeismicDevice::upload(const SeismicHost& h, int dim) {
     cuda_check(cudaStreamSynchronize(s), "sync");
 }
 
-void SeismicDevice::adopt(const std::vector<int64_t>& lbp, const std::vector<int64_t>& bdp,
+void SeismicDevice::adopt(const std::vector<int64_t>& lbp, DevArray<int64_t>&& bdp,
                           const std::vector<int64_t>& ltp, int esz, int dim,
                           DevArray<int32_t>&& docs, DevArray<uint16_t>&& sterm,
                           DevArray<int64_t>&& srun, DevArray<uint16_t>&& sblk,
@@ -304,8 +304,8 @@ void SeismicDevice::adopt(const std::vector<int64_t>& lbp, const std::vector<int
         max_blocks_ = std::max<int32_t>(max_blocks_, static_cast<int32_t>(lbp[t + 1] - lbp[t]));
     esz_ = esz;
     lbp_.upload(lbp.data(), lbp.size(), s);
-    bdp_.upload(bdp.data(), bdp.size(), s);
     ltp_.upload(ltp.data(), ltp.size(), s);
+    bdp_ = std::move(bdp);
     docs_ = std::move(docs);
     sterm_ = std::move(sterm);
     srun_ = std::move(srun);
