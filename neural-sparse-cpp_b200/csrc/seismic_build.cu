@@ -11,7 +11,8 @@
 //                   std::uniform_int_distribution<> seeded base_seed + list,
 //                   the reference's own draw (cluster/random_kmeans.cpp:28-51);
 //                   it depends only on list lengths, so only those come back.
-//  3. assignment    one CTA per list: the centroids' terms are indexed term
+//  3. assignment    uint8 codes: on the tensor cores (seismic_assign_u8.cu).
+//                   Else one CTA per list: the centroids' terms are indexed term
 //                   major in scratch, one warp per document accumulates its
 //                   similarity to every centroid in the document's term order
 //                   (cluster/kmeans_utils.cpp:131-145; fp32 products and sums
@@ -45,6 +46,7 @@
 #include "ref_order.h"
 #include "scan.h"
 #include "segsort.cuh"
+#include "seismic_assign_u8.h"
 #include "seismic_summaries.h"
 
 namespace nsparse {
@@ -286,6 +288,11 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
         const int32_t nc = static_cast<int32_t>(a.cptr[t + 1] - a.cptr[t]);
         if (n == 0) continue;
         const int32_t* cp = a.cpos + a.cptr[t];
+        if (n == nc) {  // every doc is a centroid
+            for (int32_t c = threadIdx.x; c < nc; c += blockDim.x)
+                a.out_key[kb + cp[c]] = static_cast<uint32_t>(c) * 2u;
+            continue;
+        }
         for (int32_t i = threadIdx.x; i < n; i += blockDim.x) isc[i] = 0;
         if (threadIdx.x == 0) {
             s_touched = 0;
@@ -632,11 +639,19 @@ void build_typed(SeismicState& st, int dim, const SeismicClusterParameters& p) {
     clock.mark("centroids");
     // ---- 3. assignment
     DevArray<uint32_t> akey(static_cast<size_t>(std::max<int64_t>(total_kept, 1)));
-    if (total_kept > 0) {
-        // centroid entries per list bound: max_nc rows of the longest rows
-        int64_t max_row = 0;
-        for (int64_t d = 0; d < n_docs; ++d)
-            max_row = std::max<int64_t>(max_row, h.indptr[d + 1] - h.indptr[d]);
+    // centroid entries per list bound: max_nc rows of the longest rows
+    int64_t max_row = 0;
+    for (int64_t d = 0; d < n_docs; ++d)
+        max_row = std::max<int64_t>(max_row, h.indptr[d + 1] - h.indptr[d]);
+    bool assigned = total_kept == 0;
+    if (ESZ == 1 && !assigned) {
+        const nsp::AssignLists lists{n_lists,       d_kept_ptr.data(), kept.data(), d_cptr.data(),
+                                     d_cpos.data(), max_nc,            max_kept,    max_row};
+        std::vector<int64_t> df(static_cast<size_t>(n_lists));
+        for (int32_t t = 0; t < n_lists; ++t) df[t] = h_post[t + 1] - h_post[t];
+        assigned = nsp::assign_u8(f, lists, df, akey.data(), s);
+    }
+    if (!assigned) {
         const int64_t max_ce = std::max<int64_t>(1, static_cast<int64_t>(max_nc) * max_row);
         const int wpb = 32;
         const size_t acc_bytes = sizeof(assign_acc_t<ESZ>);
