@@ -42,6 +42,37 @@ static int max_smem_optin() {
     return v;
 }
 
+// ---------------------------------------------------------------- arena --
+
+Arena::~Arena() {
+    if (chunks_.empty()) return;
+    cudaStreamSynchronize(s_);
+    for (const Chunk& c : chunks_) cudaFree(c.p);
+}
+
+void* Arena::bytes(size_t n) {
+    n = (n + 255) & ~size_t(255);
+    while (cur_ < chunks_.size() && used_ + n > chunks_[cur_].cap) {
+        ++cur_;
+        used_ = 0;
+    }
+    if (cur_ == chunks_.size()) {
+        // each chunk twice the one before, 64 MB to 1 GB, so a small build
+        // holds little and a large one needs few
+        size_t cap = size_t{64} << 20;
+        if (!chunks_.empty())
+            cap = std::min(std::max(cap, 2 * chunks_.back().cap), size_t{1} << 30);
+        cap = std::max(cap, n);
+        void* p = nullptr;
+        cuda_check(cudaMalloc(&p, cap), "arena cudaMalloc");
+        chunks_.push_back({static_cast<char*>(p), cap});
+        used_ = 0;
+    }
+    void* p = chunks_[cur_].p + used_;
+    used_ += n;
+    return p;
+}
+
 // ------------------------------------------------------------ workspace --
 
 Workspace::Workspace() {
@@ -158,21 +189,19 @@ void ForwardDevice::upload(const HostCsr& h) {
         return;
     }
     const int64_t nnz = h.nnz();
-    DevArray<int32_t> d_indptr;
-    DevArray<uint16_t> d_idx;
-    DevArray<uint8_t> d_val;
-    d_indptr.upload(h.indptr.data(), h.indptr.size(), s);
-    d_idx.upload(h.indices.data(), static_cast<size_t>(nnz), s);
-    d_val.upload(h.values.data(), static_cast<size_t>(nnz) * esz_, s);
-    DevArray<int64_t> units(static_cast<size_t>(n_docs_) + 1);
+    Arena scratch(s);
+    const int32_t* d_indptr = scratch.put(h.indptr.data(), h.indptr.size());
+    const uint16_t* d_idx = scratch.put(h.indices.data(), static_cast<size_t>(nnz));
+    const uint8_t* d_val = scratch.put(h.values.data(), static_cast<size_t>(nnz) * esz_);
+    int64_t* units = scratch.take<int64_t>(static_cast<size_t>(n_docs_) + 1);
     row_units_kernel<<<std::min<int64_t>((n_docs_ + 255) / 256, 148 * 16), 256, 0, s>>>(
-        d_indptr.data(), n_docs_, units.data());
+        d_indptr, n_docs_, units);
     cuda_check(cudaGetLastError(), "row_units_kernel");
     // exclusive scan in place over n+1 entries (last entry = total units)
-    cuda_check(cudaMemsetAsync(units.data() + n_docs_, 0, sizeof(int64_t), s), "memset");
-    exclusive_scan_i64(units.data(), units.data(), static_cast<int64_t>(n_docs_) + 1, s);
+    cuda_check(cudaMemsetAsync(units + n_docs_, 0, sizeof(int64_t), s), "memset");
+    exclusive_scan_i64(units, units, static_cast<int64_t>(n_docs_) + 1, s, scratch);
     int64_t total_units = 0;
-    cuda_check(cudaMemcpyAsync(&total_units, units.data() + n_docs_, sizeof(int64_t),
+    cuda_check(cudaMemcpyAsync(&total_units, units + n_docs_, sizeof(int64_t),
                                cudaMemcpyDeviceToHost, s), "D2H");
     cuda_check(cudaStreamSynchronize(s), "sync");
     if (total_units > static_cast<int64_t>(UINT32_MAX))
@@ -181,8 +210,8 @@ void ForwardDevice::upload(const HostCsr& h) {
     rowinfo_.resize(static_cast<size_t>(n_docs_));
     idx_.resize(std::max<size_t>(padded, 16));
     val_.resize(std::max<size_t>(padded * esz_, 16));
-    pad_rows_kernel<<<148 * 16, 256, 0, s>>>(d_indptr.data(), d_idx.data(), d_val.data(), n_docs_,
-                                             esz_, units.data(), rowinfo_.data(), idx_.data(),
+    pad_rows_kernel<<<148 * 16, 256, 0, s>>>(d_indptr, d_idx, d_val, n_docs_,
+                                             esz_, units, rowinfo_.data(), idx_.data(),
                                              val_.data());
     cuda_check(cudaGetLastError(), "pad_rows_kernel");
     cuda_check(cudaStreamSynchronize(s), "sync");

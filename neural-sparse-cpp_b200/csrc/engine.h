@@ -77,6 +77,50 @@ private:
     size_t n_ = 0;
 };
 
+// Device scratch of one operation on one stream: bump allocation from a few
+// large cudaMalloc chunks, given back when the operation ends. A build of
+// 200,000 docs made about 60 allocations; each cudaMalloc / cudaFree pair
+// costs 0.7-1.1 ms, up to 100 ms when the machine's other GPUs allocate at the
+// same time. Memory released back to a mark is reused in stream order.
+class Arena {
+public:
+    explicit Arena(cudaStream_t s) : s_(s) {}
+    ~Arena();
+    Arena(const Arena&) = delete;
+    Arena& operator=(const Arena&) = delete;
+    // At least one element, 256-byte aligned, contents undefined.
+    template <class T>
+    T* take(size_t n) {
+        return static_cast<T*>(bytes((n > 0 ? n : 1) * sizeof(T)));
+    }
+    // A copy of host memory (the source may be reused on return).
+    template <class T>
+    T* put(const T* h, size_t n) {
+        T* d = take<T>(n);
+        if (n > 0)
+            cuda_check(cudaMemcpyAsync(d, h, n * sizeof(T), cudaMemcpyHostToDevice, s_), "H2D");
+        return d;
+    }
+    struct Mark {
+        size_t chunk, used;
+    };
+    Mark mark() const { return {cur_, used_}; }
+    void release(Mark m) {
+        cur_ = m.chunk;
+        used_ = m.used;
+    }
+
+private:
+    void* bytes(size_t n);
+    struct Chunk {
+        char* p;
+        size_t cap;
+    };
+    cudaStream_t s_;
+    std::vector<Chunk> chunks_;
+    size_t cur_ = 0, used_ = 0;
+};
+
 // Device scratch by slot, grow-only: the per-thread Workspace, or the
 // buffers a captured search graph owns.
 class Scratch {

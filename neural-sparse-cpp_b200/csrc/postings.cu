@@ -129,58 +129,59 @@ void PostingsDevice::build(const ForwardDevice& fwd, int chunk_docs) {
     const FwdView f = fwd.view();
     const int32_t n = f.n_docs;
 
-    DevArray<int64_t> off(static_cast<size_t>(n) + 1);
-    DevArray<int> flag(1);
-    cuda_check(cudaMemsetAsync(flag.data(), 0, sizeof(int), s), "memset");
-    cuda_check(cudaMemsetAsync(off.data() + n, 0, sizeof(int64_t), s), "memset");
-    row_lens_kernel<<<grid_for(static_cast<int64_t>(n) * 32, 256), 256, 0, s>>>(f, off.data(),
-                                                                                flag.data());
+    Arena scratch(s);
+    int64_t* off = scratch.take<int64_t>(static_cast<size_t>(n) + 1);
+    int* flag = scratch.take<int>(1);
+    cuda_check(cudaMemsetAsync(flag, 0, sizeof(int), s), "memset");
+    cuda_check(cudaMemsetAsync(off + n, 0, sizeof(int64_t), s), "memset");
+    row_lens_kernel<<<grid_for(static_cast<int64_t>(n) * 32, 256), 256, 0, s>>>(f, off,
+                                                                                flag);
     cuda_check(cudaGetLastError(), "row_lens_kernel");
-    exclusive_scan_i64(off.data(), off.data(), static_cast<int64_t>(n) + 1, s);
+    exclusive_scan_i64(off, off, static_cast<int64_t>(n) + 1, s, scratch);
     int64_t nnz = 0;
     int unsorted = 0;
-    cuda_check(cudaMemcpyAsync(&nnz, off.data() + n, sizeof(nnz), cudaMemcpyDeviceToHost, s), "D2H");
-    cuda_check(cudaMemcpyAsync(&unsorted, flag.data(), sizeof(int), cudaMemcpyDeviceToHost, s),
+    cuda_check(cudaMemcpyAsync(&nnz, off + n, sizeof(nnz), cudaMemcpyDeviceToHost, s), "D2H");
+    cuda_check(cudaMemcpyAsync(&unsorted, flag, sizeof(int), cudaMemcpyDeviceToHost, s),
                "D2H");
     cuda_check(cudaStreamSynchronize(s), "sync");
     if (unsorted != 0 || nnz >= INT_MAX) return;  // the tile kernel serves this index
 
     n_chunks_ = (n + chunk_docs - 1) / chunk_docs;
     const int dim = f.dim;
-    DevArray<int32_t> tstart(static_cast<size_t>(dim) + 1);
+    int32_t* tstart = scratch.take<int32_t>(static_cast<size_t>(dim) + 1);
     doc_.resize(static_cast<size_t>(std::max<int64_t>(nnz, 1)));
     val_.resize(static_cast<size_t>(std::max<int64_t>(nnz, 1)));
     if (nnz > 0) {
-        DevArray<uint16_t> k_in(static_cast<size_t>(nnz)), k_out(static_cast<size_t>(nnz));
-        DevArray<unsigned long long> v_in(static_cast<size_t>(nnz)), v_out(static_cast<size_t>(nnz));
+        uint16_t* k_in = scratch.take<uint16_t>(static_cast<size_t>(nnz));
+        uint16_t* k_out = scratch.take<uint16_t>(static_cast<size_t>(nnz));
+        auto* v_in = scratch.take<unsigned long long>(static_cast<size_t>(nnz));
+        auto* v_out = scratch.take<unsigned long long>(static_cast<size_t>(nnz));
         compact_kernel<<<grid_for(static_cast<int64_t>(n) * 32, 256), 256, 0, s>>>(
-            f, off.data(), k_in.data(), v_in.data());
+            f, off, k_in, v_in);
         cuda_check(cudaGetLastError(), "compact_kernel");
         size_t tmp_bytes = 0;
-        cuda_check(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, k_in.data(), k_out.data(),
-                                                   v_in.data(), v_out.data(), static_cast<int>(nnz),
+        cuda_check(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, k_in, k_out,
+                                                   v_in, v_out, static_cast<int>(nnz),
                                                    0, 16, s),
                    "radix sort size");
-        DevArray<unsigned char> tmp(std::max<size_t>(tmp_bytes, 1));
-        cuda_check(cub::DeviceRadixSort::SortPairs(tmp.data(), tmp_bytes, k_in.data(), k_out.data(),
-                                                   v_in.data(), v_out.data(), static_cast<int>(nnz),
+        auto* tmp = scratch.take<unsigned char>(tmp_bytes);
+        cuda_check(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, k_in, k_out,
+                                                   v_in, v_out, static_cast<int>(nnz),
                                                    0, 16, s),
                    "radix sort");
-        term_start_kernel<<<(dim + 1 + 255) / 256, 256, 0, s>>>(k_out.data(), nnz, dim,
-                                                                tstart.data());
+        term_start_kernel<<<(dim + 1 + 255) / 256, 256, 0, s>>>(k_out, nnz, dim,
+                                                                tstart);
         cuda_check(cudaGetLastError(), "term_start_kernel");
-        unpack_kernel<<<grid_for(nnz, 256), 256, 0, s>>>(v_out.data(), nnz, doc_.data(),
+        unpack_kernel<<<grid_for(nnz, 256), 256, 0, s>>>(v_out, nnz, doc_.data(),
                                                          val_.data());
         cuda_check(cudaGetLastError(), "unpack_kernel");
-        // the temporaries are freed when this scope ends: wait for their users
-        cuda_check(cudaStreamSynchronize(s), "sync");
     } else {
-        cuda_check(cudaMemsetAsync(tstart.data(), 0, (static_cast<size_t>(dim) + 1) * 4, s),
+        cuda_check(cudaMemsetAsync(tstart, 0, (static_cast<size_t>(dim) + 1) * 4, s),
                    "memset");
     }
     chunk_at_.resize(static_cast<size_t>(dim) * (n_chunks_ + 1));
     chunk_at_kernel<<<grid_for(static_cast<int64_t>(dim) * (n_chunks_ + 1), 256), 256, 0, s>>>(
-        tstart.data(), doc_.data(), dim, n_chunks_, chunk_docs, chunk_at_.data());
+        tstart, doc_.data(), dim, n_chunks_, chunk_docs, chunk_at_.data());
     cuda_check(cudaGetLastError(), "chunk_at_kernel");
     cuda_check(cudaStreamSynchronize(s), "sync");
     usable_ = true;

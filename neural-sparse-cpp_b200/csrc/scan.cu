@@ -88,17 +88,19 @@ __global__ void __launch_bounds__(kThreads) tile_scan_kernel(const int64_t* in, 
 
 }  // namespace
 
-void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t s) {
+void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t s,
+                        Arena& scratch) {
     if (n <= 0) return;
     const int64_t tiles = (n + kTile - 1) / kTile;
-    DevArray<int64_t> sums(static_cast<size_t>(tiles));
-    tile_sums_kernel<<<static_cast<unsigned>(tiles), kThreads, 0, s>>>(in, n, sums.data());
+    const Arena::Mark m = scratch.mark();
+    int64_t* sums = scratch.take<int64_t>(static_cast<size_t>(tiles));
+    tile_sums_kernel<<<static_cast<unsigned>(tiles), kThreads, 0, s>>>(in, n, sums);
     cuda_check(cudaGetLastError(), "tile_sums_kernel");
-    scan_sums_kernel<<<1, kThreads, 0, s>>>(sums.data(), tiles);
+    scan_sums_kernel<<<1, kThreads, 0, s>>>(sums, tiles);
     cuda_check(cudaGetLastError(), "scan_sums_kernel");
-    tile_scan_kernel<<<static_cast<unsigned>(tiles), kThreads, 0, s>>>(in, out, n, sums.data());
+    tile_scan_kernel<<<static_cast<unsigned>(tiles), kThreads, 0, s>>>(in, out, n, sums);
     cuda_check(cudaGetLastError(), "tile_scan_kernel");
-    cuda_check(cudaStreamSynchronize(s), "scan sync");
+    scratch.release(m);
 }
 
 }  // namespace nsp

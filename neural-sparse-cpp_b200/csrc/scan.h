@@ -9,9 +9,12 @@
 
 namespace nsp {
 
-// out[i] = sum(in[0..i)); in and out may alias. Synchronous with respect to
-// the host only where it allocates its block-sum scratch.
-void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t s);
+class Arena;
+
+// out[i] = sum(in[0..i)); in and out may alias. Its block sums come from
+// `scratch` (an arena of the same stream) and go back to it.
+void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t s,
+                        Arena& scratch);
 
 }  // namespace nsp
 

@@ -556,7 +556,7 @@ hot_rows_kernel(FwdView f, const uint16_t* slot_of, int hot_bytes, uint8_t* hot,
 }  // namespace
 
 bool assign_u8(const FwdView& f, const AssignLists& lists, const std::vector<int64_t>& df,
-               uint32_t* out_key, cudaStream_t s) {
+               uint32_t* out_key, cudaStream_t s, Arena& scratch) {
     const int dim = f.dim;
     if (lists.max_nc > kAssignMaxCentroids || f.n_docs == 0 || dim > kMaxDim) return false;
     // the hot terms: as many as the dense rows hold, by document frequency
@@ -589,49 +589,47 @@ bool assign_u8(const FwdView& f, const AssignLists& lists, const std::vector<int
         bits[t >> 5] |= 1u << (t & 31);
     }
     const int sms = device_sm_count();
-    DevArray<uint16_t> d_slot;
-    DevArray<uint32_t> d_bits;
-    d_slot.upload(slot_of.data(), slot_of.size(), s);
-    d_bits.upload(bits.data(), bits.size(), s);
-    DevArray<uint8_t> hot(static_cast<size_t>(f.n_docs) * hot_bytes);
-    DevArray<int32_t> flags(3);  // unsorted rows, list counter, error
-    cuda_check(cudaMemsetAsync(flags.data(), 0, 3 * sizeof(int32_t), s), "memset");
-    hot_rows_kernel<<<sms * 8, kRowWarps * 32, 0, s>>>(f, d_slot.data(), hot_bytes, hot.data(),
-                                                       flags.data());
+    const Arena::Mark mark = scratch.mark();
+    const uint16_t* d_slot = scratch.put(slot_of.data(), slot_of.size());
+    const uint32_t* d_bits = scratch.put(bits.data(), bits.size());
+    uint8_t* hot = scratch.take<uint8_t>(static_cast<size_t>(f.n_docs) * hot_bytes);
+    int32_t* flags = scratch.take<int32_t>(3);  // unsorted rows, list counter, error
+    cuda_check(cudaMemsetAsync(flags, 0, 3 * sizeof(int32_t), s), "memset");
+    hot_rows_kernel<<<sms * 8, kRowWarps * 32, 0, s>>>(f, d_slot, hot_bytes, hot, flags);
     cuda_check(cudaGetLastError(), "hot_rows_kernel");
     int32_t unsorted = 0;
-    cuda_check(cudaMemcpyAsync(&unsorted, flags.data(), sizeof(unsorted), cudaMemcpyDeviceToHost,
+    cuda_check(cudaMemcpyAsync(&unsorted, flags, sizeof(unsorted), cudaMemcpyDeviceToHost,
                                s), "D2H");
     cuda_check(cudaStreamSynchronize(s), "sync");
-    if (unsorted != 0) return false;
+    if (unsorted != 0) {
+        scratch.release(mark);
+        return false;
+    }
 
     const int ctas = sms;
     const int64_t max_entries = std::max<int64_t>(1, static_cast<int64_t>(lists.max_nc) *
                                                          lists.max_row);
     const int64_t max_kept = std::max<int64_t>(lists.max_kept, 1);
     const size_t n = static_cast<size_t>(ctas);
-    DevArray<int32_t> ends(n * (dim + 1)), member(n * max_kept);
-    DevArray<uint32_t> entry(n * max_entries);
-    DevArray<uint8_t> isc(n * max_kept);
+    int32_t* ends = scratch.take<int32_t>(n * (dim + 1));
     // a pass's centroids are padded to 16, so up to 4 passes fill 1,088 columns
     const int ld = kAssignMaxCentroids + 64;
-    DevArray<int32_t> sims(n * kM * ld);
-    cuda_check(cudaMemsetAsync(ends.data(), 0, ends.size() * sizeof(int32_t), s), "memset");
+    cuda_check(cudaMemsetAsync(ends, 0, n * (dim + 1) * sizeof(int32_t), s), "memset");
     Args a{};
     a.f = f;
     a.l = lists;
-    a.hot = hot.data();
+    a.hot = hot;
     a.hot_bytes = hot_bytes;
-    a.hot_bits = d_bits.data();
+    a.hot_bits = d_bits;
     a.words = words;
     a.out_key = out_key;
-    a.work = flags.data() + 1;
-    a.err = flags.data() + 2;
-    a.ends = ends.data();
-    a.entry = entry.data();
-    a.member = member.data();
-    a.is_centroid = isc.data();
-    a.sims = sims.data();
+    a.work = flags + 1;
+    a.err = flags + 2;
+    a.ends = ends;
+    a.entry = scratch.take<uint32_t>(n * max_entries);
+    a.member = scratch.take<int32_t>(n * max_kept);
+    a.is_centroid = scratch.take<uint8_t>(n * max_kept);
+    a.sims = scratch.take<int32_t>(n * kM * ld);
     a.max_entries = max_entries;
     a.max_kept = max_kept;
     a.ld = ld;
@@ -644,6 +642,7 @@ bool assign_u8(const FwdView& f, const AssignLists& lists, const std::vector<int
     int32_t err = 0;
     cuda_check(cudaMemcpyAsync(&err, a.err, sizeof(err), cudaMemcpyDeviceToHost, s), "D2H");
     cuda_check(cudaStreamSynchronize(s), "assign sync");
+    scratch.release(mark);
     if (err != 0) throw std::runtime_error("assignment kernel gave up waiting for the tensor core");
     return true;
 }

@@ -31,7 +31,7 @@ struct AssignLists {
 // less than half of the products.
 constexpr int kAssignMaxCentroids = 1024;
 bool assign_u8(const FwdView& f, const AssignLists& lists, const std::vector<int64_t>& df,
-               uint32_t* out_key, cudaStream_t s);
+               uint32_t* out_key, cudaStream_t s, Arena& scratch);
 
 }  // namespace nsp
 

@@ -452,16 +452,11 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
 }
 
 template <class T>
-std::vector<T> to_host(const DevArray<T>& d, size_t n, cudaStream_t s) {
+std::vector<T> to_host(const T* d, size_t n, cudaStream_t s) {
     std::vector<T> h(n);
-    d.download(h.data(), n, s);
+    cuda_check(cudaMemcpyAsync(h.data(), d, n * sizeof(T), cudaMemcpyDeviceToHost, s), "D2H");
     cuda_check(cudaStreamSynchronize(s), "D2H");
     return h;
-}
-
-template <class T>
-void to_dev(DevArray<T>& d, const std::vector<T>& h, cudaStream_t s) {
-    d.upload(h.data(), h.size(), s);
 }
 
 std::vector<int32_t> to_i32_offsets(const std::vector<int64_t>& v) {
@@ -503,7 +498,7 @@ __global__ void block_bounds_kernel(const uint32_t* key, const int64_t* kept_ptr
 // (value desc, then doc asc) is already the reference's.
 void reference_tie_order(const nsp::HostCsr& h, const std::vector<int64_t>& post,
                          const std::vector<int64_t>& kept_ptr, const std::vector<uint8_t>& tie,
-                         int64_t cap, DevArray<int32_t>& kept, cudaStream_t s) {
+                         int64_t cap, int32_t* kept, cudaStream_t s) {
     std::vector<int32_t> lists;
     for (int32_t t = 0; t < static_cast<int32_t>(tie.size()); ++t)
         if (tie[t]) lists.push_back(t);
@@ -511,7 +506,7 @@ void reference_tie_order(const nsp::HostCsr& h, const std::vector<int64_t>& post
     std::vector<int32_t> out;
     nsp::reference_kept_order(h, post, lists, cap, out);
     for (size_t j = 0; j < lists.size(); ++j)
-        cuda_check(cudaMemcpyAsync(kept.data() + kept_ptr[lists[j]], out.data() + j * cap,
+        cuda_check(cudaMemcpyAsync(kept + kept_ptr[lists[j]], out.data() + j * cap,
                                    static_cast<size_t>(cap) * sizeof(int32_t),
                                    cudaMemcpyHostToDevice, s),
                    "H2D kept order");
@@ -555,26 +550,17 @@ void build_typed(SeismicState& st, int dim, const SeismicClusterParameters& p) {
     PhaseClock clock(s);
 
     // ---- 1. postings
-    DevArray<unsigned long long> cnt(static_cast<size_t>(n_lists) + 1);
-    cuda_check(cudaMemsetAsync(cnt.data(), 0, cnt.size() * 8, s), "memset");
-    post_count_kernel<<<sms * 8, 256, 0, s>>>(f, cnt.data());
+    nsp::Arena arena(s);
+    const size_t nl1 = static_cast<size_t>(n_lists) + 1;
+    auto* cnt = arena.take<unsigned long long>(nl1);
+    cuda_check(cudaMemsetAsync(cnt, 0, nl1 * 8, s), "memset");
+    post_count_kernel<<<sms * 8, 256, 0, s>>>(f, cnt);
     cuda_check(cudaGetLastError(), "post_count_kernel");
-    DevArray<int64_t> post_ptr(static_cast<size_t>(n_lists) + 1);
-    nsp::exclusive_scan_i64(reinterpret_cast<const int64_t*>(cnt.data()), post_ptr.data(),
-                            n_lists + 1, s);
+    int64_t* post_ptr = arena.take<int64_t>(nl1);
+    nsp::exclusive_scan_i64(reinterpret_cast<const int64_t*>(cnt), post_ptr, n_lists + 1, s,
+                            arena);
     const std::vector<int64_t> h_post = to_host(post_ptr, n_lists + 1, s);
     const int64_t nnz = h_post.back();
-    DevArray<uint64_t> keys(static_cast<size_t>(std::max<int64_t>(nnz, 1)));
-    DevArray<uint64_t> keys2(static_cast<size_t>(std::max<int64_t>(nnz, 1)));
-    cuda_check(cudaMemsetAsync(cnt.data(), 0, cnt.size() * 8, s), "memset");
-    post_scatter_kernel<ESZ><<<sms * 8, 256, 0, s>>>(f, post_ptr.data(), cnt.data(), cap, keys.data());
-    cuda_check(cudaGetLastError(), "post_scatter_kernel");
-    {
-        DevArray<int32_t> off32;
-        to_dev(off32, to_i32_offsets(h_post), s);
-        segmented_sort_keys(keys.data(), keys2.data(), nnz, n_lists, off32.data(), s);
-    }
-    keys.reset();
     std::vector<int32_t> kept_len(n_lists);
     std::vector<int64_t> kept_ptr(n_lists + 1, 0);
     for (int32_t t = 0; t < n_lists; ++t) {
@@ -583,26 +569,29 @@ void build_typed(SeismicState& st, int dim, const SeismicClusterParameters& p) {
         kept_ptr[t + 1] = kept_ptr[t] + kept_len[t];
     }
     const int64_t total_kept = kept_ptr.back();
-    DevArray<int64_t> d_kept_ptr;
-    to_dev(d_kept_ptr, kept_ptr, s);
-    DevArray<int32_t> kept(static_cast<size_t>(std::max<int64_t>(total_kept, 1)));
-    kept_copy_kernel<<<sms * 8, 256, 0, s>>>(keys2.data(), post_ptr.data(), d_kept_ptr.data(),
-                                             n_lists, kept.data());
-    cuda_check(cudaGetLastError(), "kept_copy_kernel");
-    std::vector<uint8_t> tie(static_cast<size_t>(n_lists), 0);
-    if (ESZ == 4 && cap > 0) {
-        DevArray<uint8_t> d_tie(static_cast<size_t>(n_lists));
-        tie_flag_kernel<<<sms * 8, 256, 0, s>>>(keys2.data(), post_ptr.data(), n_lists, cap,
-                                                d_tie.data());
-        cuda_check(cudaGetLastError(), "tie_flag_kernel");
-        d_tie.download(tie.data(), tie.size(), s);
+    const int64_t* d_kept_ptr = arena.put(kept_ptr.data(), nl1);
+    int32_t* kept = arena.take<int32_t>(static_cast<size_t>(total_kept));
+    const nsp::Arena::Mark before_keys = arena.mark();
+    uint64_t* keys = arena.take<uint64_t>(static_cast<size_t>(nnz));
+    uint64_t* keys2 = arena.take<uint64_t>(static_cast<size_t>(nnz));
+    cuda_check(cudaMemsetAsync(cnt, 0, nl1 * 8, s), "memset");
+    post_scatter_kernel<ESZ><<<sms * 8, 256, 0, s>>>(f, post_ptr, cnt, cap, keys);
+    cuda_check(cudaGetLastError(), "post_scatter_kernel");
+    {
+        const std::vector<int32_t> off32 = to_i32_offsets(h_post);
+        segmented_sort_keys(keys, keys2, nnz, n_lists, arena.put(off32.data(), nl1), s, arena);
     }
-    cuda_check(cudaStreamSynchronize(s), "sync");
-    keys2.reset();
-    if (ESZ == 4) reference_tie_order(h, h_post, kept_ptr, tie, cap, kept, s);
+    kept_copy_kernel<<<sms * 8, 256, 0, s>>>(keys2, post_ptr, d_kept_ptr, n_lists, kept);
+    cuda_check(cudaGetLastError(), "kept_copy_kernel");
+    uint8_t* d_tie = nullptr;
+    if (ESZ == 4 && cap > 0) {
+        d_tie = arena.take<uint8_t>(static_cast<size_t>(n_lists));
+        tie_flag_kernel<<<sms * 8, 256, 0, s>>>(keys2, post_ptr, n_lists, cap, d_tie);
+        cuda_check(cudaGetLastError(), "tie_flag_kernel");
+    }
 
-    clock.mark("postings");
-    // ---- 2. centroid positions (host; depends on list lengths only)
+    // ---- 2. centroid positions (host; depends on list lengths only, so the
+    // device sorts the postings meanwhile)
     std::vector<int64_t> cptr(n_lists + 1, 0);
     for (int32_t t = 0; t < n_lists; ++t)
         cptr[t + 1] = cptr[t] + (kept_len[t] > 0 ? static_cast<int64_t>(clusters_for(kept_len[t], beta)) : 0);
@@ -631,25 +620,27 @@ void build_typed(SeismicState& st, int dim, const SeismicClusterParameters& p) {
         }
         for (auto& th : pool) th.join();
     }
-    DevArray<int64_t> d_cptr;
-    DevArray<int32_t> d_cpos;
-    to_dev(d_cptr, cptr, s);
-    to_dev(d_cpos, cpos, s);
+    std::vector<uint8_t> tie(static_cast<size_t>(n_lists), 0);
+    if (d_tie != nullptr) tie = to_host(d_tie, tie.size(), s);
+    arena.release(before_keys);
+    if (ESZ == 4) reference_tie_order(h, h_post, kept_ptr, tie, cap, kept, s);
+    const int64_t* d_cptr = arena.put(cptr.data(), nl1);
+    const int32_t* d_cpos = arena.put(cpos.data(), cpos.size());
 
-    clock.mark("centroids");
+    clock.mark("postings, centroids");
     // ---- 3. assignment
-    DevArray<uint32_t> akey(static_cast<size_t>(std::max<int64_t>(total_kept, 1)));
+    uint32_t* akey = arena.take<uint32_t>(static_cast<size_t>(total_kept));
     // centroid entries per list bound: max_nc rows of the longest rows
     int64_t max_row = 0;
     for (int64_t d = 0; d < n_docs; ++d)
         max_row = std::max<int64_t>(max_row, h.indptr[d + 1] - h.indptr[d]);
     bool assigned = total_kept == 0;
     if (ESZ == 1 && !assigned) {
-        const nsp::AssignLists lists{n_lists,       d_kept_ptr.data(), kept.data(), d_cptr.data(),
-                                     d_cpos.data(), max_nc,            max_kept,    max_row};
+        const nsp::AssignLists lists{n_lists, d_kept_ptr, kept,     d_cptr,
+                                     d_cpos,  max_nc,     max_kept, max_row};
         std::vector<int64_t> df(static_cast<size_t>(n_lists));
         for (int32_t t = 0; t < n_lists; ++t) df[t] = h_post[t + 1] - h_post[t];
-        assigned = nsp::assign_u8(f, lists, df, akey.data(), s);
+        assigned = nsp::assign_u8(f, lists, df, akey, s, arena);
     }
     if (!assigned) {
         const int64_t max_ce = std::max<int64_t>(1, static_cast<int64_t>(max_nc) * max_row);
@@ -667,77 +658,63 @@ void build_typed(SeismicState& st, int dim, const SeismicClusterParameters& p) {
         cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, assign_kernel<ESZ>,
                                                                  wpb * 32, smem),
                    "assign occupancy");
-        const int ctas = sms * std::max(1, std::min(per_sm, 1));
-        DevArray<int32_t> tcnt(static_cast<size_t>(ctas) * dim), tstart(static_cast<size_t>(ctas) * dim),
-            tcur(static_cast<size_t>(ctas) * dim), touched(static_cast<size_t>(ctas) * max_ce);
-        DevArray<int2> trun(static_cast<size_t>(ctas) * dim);
-        DevArray<uint16_t> ccl(static_cast<size_t>(ctas) * max_ce);
-        DevArray<uint8_t> cw(static_cast<size_t>(ctas) * max_ce * ESZ);
-        DevArray<uint8_t> isc(static_cast<size_t>(ctas) * std::max<int64_t>(max_kept, 1));
-        DevArray<uint8_t> sims(static_cast<size_t>(ctas) * wpb * std::max(max_nc, 1) * 8);
-        DevArray<int32_t> work(1);
-        cuda_check(cudaMemsetAsync(tcnt.data(), 0, tcnt.size() * 4, s), "memset");
-        cuda_check(cudaMemsetAsync(trun.data(), 0, trun.size() * sizeof(int2), s), "memset");
-        cuda_check(cudaMemsetAsync(work.data(), 0, 4, s), "memset");
+        const size_t ctas = static_cast<size_t>(sms) * std::max(1, std::min(per_sm, 1));
+        const nsp::Arena::Mark mark = arena.mark();
         AssignArgs a{};
         a.f = f;
         a.n_lists = n_lists;
-        a.kept_ptr = d_kept_ptr.data();
-        a.kept = kept.data();
-        a.cptr = d_cptr.data();
-        a.cpos = d_cpos.data();
-        a.out_key = akey.data();
-        a.work = work.data();
-        a.tcnt = tcnt.data();
-        a.tstart = tstart.data();
-        a.tcur = tcur.data();
-        a.trun = trun.data();
-        a.touched = touched.data();
-        a.ccl = ccl.data();
-        a.cw = cw.data();
-        a.is_centroid = isc.data();
-        a.sims = sims.data();
+        a.kept_ptr = d_kept_ptr;
+        a.kept = kept;
+        a.cptr = d_cptr;
+        a.cpos = d_cpos;
+        a.out_key = akey;
         a.max_centroid_entries = max_ce;
         a.max_kept = std::max<int64_t>(max_kept, 1);
         a.max_nc = std::max(max_nc, 1);
         a.sims_in_smem = sims_in_smem ? 1 : 0;
-        assign_kernel<ESZ><<<ctas, wpb * 32, smem, s>>>(a);
+        a.work = arena.take<int32_t>(1);
+        a.tcnt = arena.take<int32_t>(ctas * dim);
+        a.tstart = arena.take<int32_t>(ctas * dim);
+        a.tcur = arena.take<int32_t>(ctas * dim);
+        a.trun = arena.take<int2>(ctas * dim);
+        a.touched = arena.take<int32_t>(ctas * max_ce);
+        a.ccl = arena.take<uint16_t>(ctas * max_ce);
+        a.cw = arena.take<uint8_t>(ctas * max_ce * ESZ);
+        a.is_centroid = arena.take<uint8_t>(ctas * a.max_kept);
+        a.sims = arena.take<uint8_t>(ctas * wpb * a.max_nc * 8);
+        cuda_check(cudaMemsetAsync(a.tcnt, 0, ctas * dim * 4, s), "memset");
+        cuda_check(cudaMemsetAsync(a.trun, 0, ctas * dim * sizeof(int2), s), "memset");
+        cuda_check(cudaMemsetAsync(a.work, 0, 4, s), "memset");
+        assign_kernel<ESZ><<<static_cast<unsigned>(ctas), wpb * 32, smem, s>>>(a);
         cuda_check(cudaGetLastError(), "assign_kernel");
-        cuda_check(cudaStreamSynchronize(s), "assign sync");
+        arena.release(mark);
     }
 
     clock.mark("assignment");
     // ---- 4. blocks: centroid first, members in list order
+    // (the per-block and per-posting arrays are the index's own)
     DevArray<int32_t> bdocs(static_cast<size_t>(std::max<int64_t>(total_kept, 1)));
-    DevArray<uint32_t> akey2(static_cast<size_t>(std::max<int64_t>(total_kept, 1)));
+    uint32_t* akey2 = arena.take<uint32_t>(static_cast<size_t>(total_kept));
     {
-        DevArray<int32_t> off32;
-        to_dev(off32, to_i32_offsets(kept_ptr), s);
-        segmented_sort_pairs(akey.data(), akey2.data(), kept.data(), bdocs.data(), total_kept,
-                             n_lists, off32.data(), s, /*stable=*/true);
+        const std::vector<int32_t> off32 = to_i32_offsets(kept_ptr);
+        segmented_sort_pairs(akey, akey2, kept, bdocs.data(), total_kept, n_lists,
+                             arena.put(off32.data(), nl1), s, /*stable=*/true, arena);
     }
     // one block per centroid, block docs where the sorted keys change cluster
     const int64_t n_blocks = cptr.back();
     DevArray<int64_t> bdp(static_cast<size_t>(n_blocks) + 1);
-    DevArray<uint16_t> local(static_cast<size_t>(std::max<int64_t>(n_blocks, 1)));
-    block_bounds_kernel<<<sms * 8, 128, 0, s>>>(akey2.data(), d_kept_ptr.data(), d_cptr.data(),
-                                                n_lists, bdp.data(), local.data());
+    uint16_t* local = arena.take<uint16_t>(static_cast<size_t>(n_blocks));
+    block_bounds_kernel<<<sms * 8, 128, 0, s>>>(akey2, d_kept_ptr, d_cptr, n_lists, bdp.data(),
+                                                local);
     cuda_check(cudaGetLastError(), "block_bounds_kernel");
-    cuda_check(cudaStreamSynchronize(s), "sync");
-    akey.reset();
-    akey2.reset();
-    kept.reset();
 
     clock.mark("blocks");
     // ---- 5. summaries
     nsp::DevColumns cols;
-    cols.srun.resize(1);
-    cuda_check(cudaMemsetAsync(cols.srun.data(), 0, sizeof(int64_t), s), "memset");
     std::vector<int64_t> ltp{0};
     std::vector<std::pair<std::string, double>> steps;
-    const nsp::BlockSet blocks{cptr.data(),   d_cptr.data(), n_lists,
-                               bdocs.data(),  bdp.data(),    local.data()};
-    nsp::summarize_blocks(ESZ, f, blocks, p.alpha, ESZ == 4 ? &h : nullptr, s, cols, ltp,
+    const nsp::BlockSet blocks{cptr.data(), d_cptr, n_lists, bdocs.data(), bdp.data(), local};
+    nsp::summarize_blocks(ESZ, f, blocks, p.alpha, ESZ == 4 ? &h : nullptr, s, arena, cols, ltp,
                           clock.on ? &steps : nullptr);
 
     clock.mark("summaries");

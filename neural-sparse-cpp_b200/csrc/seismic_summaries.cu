@@ -941,37 +941,13 @@ __global__ void column_bounds_kernel(const int64_t* start, int64_t n_cols, int64
         srun_tail[c] = ebase + (c + 1 < n_cols ? start[c + 1] : n_kept);
 }
 
-// Appends n elements at src (device) after the first `used` of dst, growing
-// dst geometrically.
-template <class T>
-void dev_append(DevArray<T>& dst, size_t used, const T* src, size_t n, cudaStream_t s) {
-    if (used + n > dst.size()) {
-        DevArray<T> bigger(std::max(dst.size() * 2, used + n));
-        if (used > 0)
-            cuda_check(cudaMemcpyAsync(bigger.data(), dst.data(), used * sizeof(T),
-                                       cudaMemcpyDeviceToDevice, s),
-                       "D2D");
-        cuda_check(cudaStreamSynchronize(s), "sync");
-        dst = std::move(bigger);
-    }
-    if (n > 0)
-        cuda_check(cudaMemcpyAsync(dst.data() + used, src, n * sizeof(T), cudaMemcpyDeviceToDevice,
-                                   s),
-                   "D2D");
-}
-
-// Device buffers kept across batches of lists (they only grow).
-struct Pool {
-    DevArray<int64_t> keep, flag, pos, start, lcol;
-    DevArray<uint16_t> term, blk;
-    DevArray<uint32_t> okey, tkey, tkey2;
-    DevArray<float> oval, tval, tval2;
-    DevArray<int32_t> ids, tied, list_koff;
-    DevArray<uint8_t> val, sort_tmp;
-    DevArray<uint64_t> spill;
-    DevArray<unsigned> counters;
-    DevArray<uint32_t> gvals;
-    DevArray<uint16_t> gterms;
+// A batch's columns, held until all batches are done.
+struct Piece {
+    const uint16_t* term;
+    const int64_t* start;
+    const uint16_t* blk;
+    const uint8_t* val;
+    int64_t n_cols, n_kept;
 };
 
 struct Steps {
@@ -993,71 +969,77 @@ struct Steps {
     }
 };
 
-// Kept pairs of the lists [t0, t1) -- tkey, tval in P, list_koff[l] the first
-// pair of list t0 + l -- become the lists' summary columns, term-major per
-// list (build_transpose, inverted_list_clusters.cpp:230-293), appended to
-// `out`.
-void emit_columns(int esz, int32_t nl, int64_t n_kept, cudaStream_t s, Pool& P, Steps& steps,
-                  DevColumns& out, std::vector<int64_t>& ltp) {
+// Kept pairs of `nl` lists (tkey, tval; list_koff[l] the first of list l)
+// become the lists' summary columns, term-major per list (build_transpose,
+// inverted_list_clusters.cpp:230-293), in memory of `keep`.
+Piece emit_columns(int esz, int32_t nl, int64_t n_kept, const uint32_t* tkey, const float* tval,
+                   const int32_t* list_koff, size_t cols_before, cudaStream_t s, Arena& scratch,
+                   Arena& keep, Steps& steps, std::vector<int64_t>& ltp) {
     const int sms = device_sm_count();
-    const int64_t nk1 = std::max<int64_t>(n_kept, 1);
-    segmented_sort_pairs(P.tkey.data(), P.tkey2.data(), P.tval.data(), P.tval2.data(), n_kept,
-                         nl, P.list_koff.data(), s, /*stable=*/false, &P.sort_tmp);
+    const size_t nk = static_cast<size_t>(n_kept);
+    uint32_t* key = scratch.take<uint32_t>(nk);
+    float* val = scratch.take<float>(nk);
+    segmented_sort_pairs(tkey, key, tval, val, n_kept, nl, list_koff, s, /*stable=*/false, scratch);
     steps.mark("transpose sort");
-    // columns assembled on the device: block ids, values, and one run per
-    // (list, term) with its start
-    P.blk.grow(nk1);
-    P.val.grow(nk1 * esz);
-    P.flag.grow(n_kept + 1);
-    P.pos.grow(n_kept + 1);
+    // block ids, values, and one run per (list, term) with its start
+    uint16_t* blk = keep.take<uint16_t>(nk);
+    uint8_t* out_val = keep.take<uint8_t>(nk * esz);
+    int64_t* flag = scratch.take<int64_t>(nk + 1);
+    int64_t* pos = scratch.take<int64_t>(nk + 1);
+    int64_t* lcol = scratch.take<int64_t>(static_cast<size_t>(nl) + 1);
     auto* columns = esz == 4 ? columns_kernel<4> : (esz == 2 ? columns_kernel<2> : columns_kernel<1>);
-    columns<<<sms * 8, 256, 0, s>>>(P.tkey2.data(), P.tval2.data(), n_kept, P.blk.data(),
-                                    P.val.data(), P.flag.data());
+    columns<<<sms * 8, 256, 0, s>>>(key, val, n_kept, blk, out_val, flag);
     cuda_check(cudaGetLastError(), "columns_kernel");
-    list_start_kernel<<<std::max(1, (nl + 255) / 256), 256, 0, s>>>(P.list_koff.data(), nl,
-                                                                    n_kept, P.flag.data());
+    list_start_kernel<<<std::max(1, (nl + 255) / 256), 256, 0, s>>>(list_koff, nl, n_kept, flag);
     cuda_check(cudaGetLastError(), "list_start_kernel");
-    exclusive_scan_i64(P.flag.data(), P.pos.data(), n_kept + 1, s);
-    int64_t n_cols = 0;
-    cuda_check(cudaMemcpyAsync(&n_cols, P.pos.data() + n_kept, 8, cudaMemcpyDeviceToHost, s),
-               "D2H");
-    cuda_check(cudaStreamSynchronize(s), "sync");
-    P.term.grow(std::max<int64_t>(n_cols, 1));
-    P.start.grow(std::max<int64_t>(n_cols, 1));
-    P.lcol.grow(static_cast<size_t>(nl) + 1);
-    column_compact_kernel<<<sms * 8, 256, 0, s>>>(P.tkey2.data(), P.flag.data(), P.pos.data(),
-                                                  n_kept, P.term.data(), P.start.data());
-    cuda_check(cudaGetLastError(), "column_compact_kernel");
-    list_cols_kernel<<<std::max(1, (nl + 1 + 255) / 256), 256, 0, s>>>(
-        P.list_koff.data(), nl, P.pos.data(), P.lcol.data());
+    exclusive_scan_i64(flag, pos, n_kept + 1, s, scratch);
+    list_cols_kernel<<<std::max(1, (nl + 1 + 255) / 256), 256, 0, s>>>(list_koff, nl, pos, lcol);
     cuda_check(cudaGetLastError(), "list_cols_kernel");
-    // appended to the index's device columns; only the per-list column
-    // counts come back to the host
-    const size_t eb = out.n_entries, cb = out.n_cols;
-    dev_append(out.sblk, eb, P.blk.data(), static_cast<size_t>(n_kept), s);
-    dev_append(out.sval, eb * esz, P.val.data(), static_cast<size_t>(n_kept) * esz, s);
-    dev_append(out.sterm, cb, P.term.data(), static_cast<size_t>(n_cols), s);
-    if (out.srun.size() < cb + 1 + static_cast<size_t>(n_cols)) {
-        DevArray<int64_t> bigger(
-            std::max(out.srun.size() * 2, cb + 1 + static_cast<size_t>(n_cols)));
-        cuda_check(cudaMemcpyAsync(bigger.data(), out.srun.data(), (cb + 1) * sizeof(int64_t),
-                                   cudaMemcpyDeviceToDevice, s),
-                   "D2D");
-        cuda_check(cudaStreamSynchronize(s), "sync");
-        out.srun = std::move(bigger);
-    }
-    if (n_cols > 0)
-        column_bounds_kernel<<<sms * 4, 256, 0, s>>>(P.start.data(), n_cols,
-                                                     static_cast<int64_t>(eb), n_kept,
-                                                     out.srun.data() + cb + 1);
-    cuda_check(cudaGetLastError(), "column_bounds_kernel");
+    // only the per-list column counts come back to the host
     std::vector<int64_t> h_lcol(static_cast<size_t>(nl) + 1);
-    P.lcol.download(h_lcol.data(), h_lcol.size(), s);
+    cuda_check(cudaMemcpyAsync(h_lcol.data(), lcol, h_lcol.size() * 8, cudaMemcpyDeviceToHost, s),
+               "D2H");
     cuda_check(cudaStreamSynchronize(s), "D2H");
-    out.n_entries += static_cast<size_t>(n_kept);
-    out.n_cols += static_cast<size_t>(n_cols);
-    for (int32_t l = 0; l < nl; ++l) ltp.push_back(static_cast<int64_t>(cb) + h_lcol[l + 1]);
+    const int64_t n_cols = h_lcol.back();
+    uint16_t* term = keep.take<uint16_t>(static_cast<size_t>(n_cols));
+    int64_t* start = keep.take<int64_t>(static_cast<size_t>(n_cols));
+    column_compact_kernel<<<sms * 8, 256, 0, s>>>(key, flag, pos, n_kept, term, start);
+    cuda_check(cudaGetLastError(), "column_compact_kernel");
+    for (int32_t l = 0; l < nl; ++l)
+        ltp.push_back(static_cast<int64_t>(cols_before) + h_lcol[l + 1]);
     steps.mark("columns");
+    return {term, start, blk, out_val, n_cols, n_kept};
+}
+
+// The batches' columns one after another, in arrays of exactly their size.
+void join_columns(int esz, const std::vector<Piece>& pieces, cudaStream_t s, DevColumns& out) {
+    size_t cols = 0, entries = 0;
+    for (const Piece& p : pieces) {
+        cols += static_cast<size_t>(p.n_cols);
+        entries += static_cast<size_t>(p.n_kept);
+    }
+    out.sterm.resize(cols);
+    out.srun.resize(cols + 1);
+    out.sblk.resize(entries);
+    out.sval.resize(entries * esz);
+    cuda_check(cudaMemsetAsync(out.srun.data(), 0, sizeof(int64_t), s), "memset");
+    size_t cb = 0, eb = 0;
+    auto copy = [&](void* dst, const void* src, size_t bytes) {
+        if (bytes > 0)
+            cuda_check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, s), "D2D");
+    };
+    for (const Piece& p : pieces) {
+        const size_t nk = static_cast<size_t>(p.n_kept), nc = static_cast<size_t>(p.n_cols);
+        copy(out.sterm.data() + cb, p.term, nc * sizeof(uint16_t));
+        copy(out.sblk.data() + eb, p.blk, nk * sizeof(uint16_t));
+        copy(out.sval.data() + eb * esz, p.val, nk * esz);
+        if (nc > 0)
+            column_bounds_kernel<<<device_sm_count() * 4, 256, 0, s>>>(
+                p.start, p.n_cols, static_cast<int64_t>(eb), p.n_kept, out.srun.data() + cb + 1);
+        cuda_check(cudaGetLastError(), "column_bounds_kernel");
+        cb += nc;
+        eb += nk;
+    }
 }
 
 // fp32 blocks whose alpha cut falls between equal maxima keep the terms the
@@ -1123,7 +1105,8 @@ int pow2_at_least(int64_t n) {
 
 template <int ESZ>
 void summarize_typed(const FwdView& f, const BlockSet& blocks, float alpha, const HostCsr* host,
-                     cudaStream_t s, DevColumns& out, std::vector<int64_t>& ltp, Steps& steps) {
+                     cudaStream_t s, Arena& scratch, DevColumns& out, std::vector<int64_t>& ltp,
+                     Steps& steps) {
     const int sms = device_sm_count();
     const int32_t n_lists = blocks.n_lists;
     const int64_t n_blocks = blocks.lbp[n_lists];
@@ -1134,18 +1117,19 @@ void summarize_typed(const FwdView& f, const BlockSet& blocks, float alpha, cons
                "cudaDeviceGetAttribute");
 
     // scratch slots: as many pairs as a block can have
-    DevArray<int64_t> slot(static_cast<size_t>(n_blocks) + 1);
-    block_terms_kernel<<<sms * 8, 256, 0, s>>>(f, blocks.d_docs, blocks.d_bdp, n_blocks,
-                                               slot.data());
+    const Arena::Mark start = scratch.mark();
+    int64_t* slot = scratch.take<int64_t>(static_cast<size_t>(n_blocks) + 1);
+    block_terms_kernel<<<sms * 8, 256, 0, s>>>(f, blocks.d_docs, blocks.d_bdp, n_blocks, slot);
     cuda_check(cudaGetLastError(), "block_terms_kernel");
-    exclusive_scan_i64(slot.data(), slot.data(), n_blocks + 1, s);
+    exclusive_scan_i64(slot, slot, n_blocks + 1, s, scratch);
     std::vector<int64_t> h_slot(static_cast<size_t>(n_lists) + 1);
     {
-        DevArray<int64_t> at(h_slot.size());
+        int64_t* at = scratch.take<int64_t>(h_slot.size());
         gather_i64_kernel<<<std::max(1, (n_lists + 256) / 256), 256, 0, s>>>(
-            slot.data(), blocks.d_lbp, n_lists + 1, 0, at.data(), nullptr);
+            slot, blocks.d_lbp, n_lists + 1, 0, at, nullptr);
         cuda_check(cudaGetLastError(), "gather_i64_kernel");
-        at.download(h_slot.data(), h_slot.size(), s);
+        cuda_check(cudaMemcpyAsync(h_slot.data(), at, h_slot.size() * 8, cudaMemcpyDeviceToHost, s),
+                   "D2H");
         cuda_check(cudaStreamSynchronize(s), "D2H");
     }
     steps.mark("slots");
@@ -1191,15 +1175,24 @@ void summarize_typed(const FwdView& f, const BlockSet& blocks, float alpha, cons
         p.spill_cap = pow2_at_least(p.cap);
         if (ESZ != 1) spill = std::max(spill, p.groups * p.spill_cap);
     }
-    Pool P;
-    P.spill.grow(static_cast<size_t>(spill));
+    uint64_t* spill_keys = scratch.take<uint64_t>(static_cast<size_t>(spill));
+    uint32_t* gvals = nullptr;
+    uint16_t* gterms = nullptr;
     if (!shape[kTiers - 1].smem_vals) {
-        P.gvals.grow(static_cast<size_t>(shape[kTiers - 1].grid) * shape[kTiers - 1].cap);
-        P.gterms.grow(static_cast<size_t>(shape[kTiers - 1].grid) * shape[kTiers - 1].cap);
+        const size_t n = static_cast<size_t>(shape[kTiers - 1].grid) * shape[kTiers - 1].cap;
+        gvals = scratch.take<uint32_t>(n);
+        gterms = scratch.take<uint16_t>(n);
     }
-    P.counters.grow(16);
+    // counters: blocks per tier, claims per tier, tied blocks
+    constexpr int kCounters = 2 * kTiers + 1;
+    unsigned* n_ids = scratch.take<unsigned>(kCounters);
+    unsigned* claims = n_ids + kTiers;
+    unsigned* n_tied = claims + kTiers;
 
-    const int64_t budget = int64_t{1} << 28;  // scratch pairs per batch (2 GB)
+    Arena keep(s);  // the batches' columns
+    std::vector<Piece> pieces;
+    size_t cols = 0;
+    const int64_t budget = int64_t{1} << 27;  // scratch pairs per batch (1 GB)
     int32_t t0 = 0;
     while (t0 < n_lists) {
         int32_t t1 = t0 + 1;
@@ -1212,48 +1205,44 @@ void summarize_typed(const FwdView& f, const BlockSet& blocks, float alpha, cons
             t0 = t1;
             continue;
         }
-        P.okey.grow(static_cast<size_t>(pairs));
-        P.oval.grow(static_cast<size_t>(pairs));
-        P.keep.grow(static_cast<size_t>(nb) + 1);
-        P.ids.grow(static_cast<size_t>(nb) * kTiers);
-        if (host != nullptr) P.tied.grow(static_cast<size_t>(nb));
-        // counters: blocks per tier, claims per tier, tied blocks
-        cuda_check(cudaMemsetAsync(P.counters.data(), 0, 16 * sizeof(unsigned), s), "memset");
-        unsigned* n_ids = P.counters.data();
-        unsigned* claims = n_ids + kTiers;
-        unsigned* n_tied = claims + kTiers;
-        tier_kernel<<<sms * 8, 256, 0, s>>>(blocks.d_bdp, slot.data(), b0, nb, P.ids.data(), n_ids,
-                                            P.keep.data());
+        const Arena::Mark batch = scratch.mark();
+        uint32_t* okey = scratch.take<uint32_t>(static_cast<size_t>(pairs));
+        float* oval = scratch.take<float>(static_cast<size_t>(pairs));
+        int64_t* kept = scratch.take<int64_t>(static_cast<size_t>(nb) + 1);
+        int32_t* ids = scratch.take<int32_t>(static_cast<size_t>(nb) * kTiers);
+        int32_t* tied = host != nullptr ? scratch.take<int32_t>(static_cast<size_t>(nb)) : nullptr;
+        cuda_check(cudaMemsetAsync(n_ids, 0, kCounters * sizeof(unsigned), s), "memset");
+        tier_kernel<<<sms * 8, 256, 0, s>>>(blocks.d_bdp, slot, b0, nb, ids, n_ids, kept);
         cuda_check(cudaGetLastError(), "tier_kernel");
         SumArgs a{};
         a.f = f;
         a.docs = blocks.d_docs;
         a.bdp = blocks.d_bdp;
         a.local = blocks.d_local;
-        a.slot = slot.data();
+        a.slot = slot;
         a.slot0 = h_slot[t0];
         a.b0 = b0;
         a.alpha = alpha;
-        a.keep = P.keep.data();
-        a.okey = P.okey.data();
-        a.oval = P.oval.data();
-        a.tied = host != nullptr ? P.tied.data() : nullptr;
+        a.keep = kept;
+        a.okey = okey;
+        a.oval = oval;
+        a.tied = tied;
         a.n_tied = n_tied;
-        a.spill = P.spill.data();
+        a.spill = spill_keys;
         a.words = words;
         // single rows go first: those that are not ascending join the next tier
         for (int t = 0; t < kTiers; ++t) {
             const Shape& p = shape[t];
-            a.ids = P.ids.data() + static_cast<int64_t>(t) * nb;
+            a.ids = ids + static_cast<int64_t>(t) * nb;
             a.n_ids = n_ids + t;
             a.next = claims + t;
-            a.retry = P.ids.data() + nb;
+            a.retry = ids + nb;
             a.n_retry = n_ids + 1;
             a.cap = p.cap;
             a.sel_cap = p.sel;
             a.spill_cap = p.spill_cap;
-            a.gvals = p.smem_vals ? nullptr : P.gvals.data();
-            a.gterms = p.smem_vals ? nullptr : P.gterms.data();
+            a.gvals = p.smem_vals ? nullptr : gvals;
+            a.gterms = p.smem_vals ? nullptr : gterms;
             p.kernel<<<p.grid, p.warps * 32, p.smem, s>>>(a);
             cuda_check(cudaGetLastError(), "block summary kernel");
         }
@@ -1263,48 +1252,50 @@ void summarize_typed(const FwdView& f, const BlockSet& blocks, float alpha, cons
             cuda_check(cudaMemcpyAsync(&n, n_tied, sizeof(n), cudaMemcpyDeviceToHost, s), "D2H");
             cuda_check(cudaStreamSynchronize(s), "D2H");
             if (n > 0) {
-                std::vector<int32_t> tied(n);
-                P.tied.download(tied.data(), n, s);
+                std::vector<int32_t> h_tied(n);
+                cuda_check(cudaMemcpyAsync(h_tied.data(), tied, n * sizeof(int32_t),
+                                           cudaMemcpyDeviceToHost, s), "D2H");
                 cuda_check(cudaStreamSynchronize(s), "D2H");
-                settle_ties(*host, blocks, a, nb, std::move(tied), s);
+                settle_ties(*host, blocks, a, nb, std::move(h_tied), s);
             }
             steps.mark("cut ties");
         }
         // packed per list
-        exclusive_scan_i64(P.keep.data(), P.keep.data(), nb + 1, s);
-        P.list_koff.grow(static_cast<size_t>(nl) + 1);
+        exclusive_scan_i64(kept, kept, nb + 1, s, scratch);
+        int32_t* list_koff = scratch.take<int32_t>(static_cast<size_t>(nl) + 1);
         gather_i64_kernel<<<std::max(1, (nl + 256) / 256), 256, 0, s>>>(
-            P.keep.data(), blocks.d_lbp + t0, nl + 1, b0, nullptr, P.list_koff.data());
+            kept, blocks.d_lbp + t0, nl + 1, b0, nullptr, list_koff);
         cuda_check(cudaGetLastError(), "gather_i64_kernel");
         int64_t n_kept = 0;
-        cuda_check(cudaMemcpyAsync(&n_kept, P.keep.data() + nb, 8, cudaMemcpyDeviceToHost, s),
-                   "D2H");
+        cuda_check(cudaMemcpyAsync(&n_kept, kept + nb, 8, cudaMemcpyDeviceToHost, s), "D2H");
         cuda_check(cudaStreamSynchronize(s), "D2H");
-        const size_t nk1 = static_cast<size_t>(std::max<int64_t>(n_kept, 1));
-        P.tkey.grow(nk1);
-        P.tkey2.grow(nk1);
-        P.tval.grow(nk1);
-        P.tval2.grow(nk1);
-        pack_pairs_kernel<<<sms * 16, 256, 0, s>>>(slot.data(), a.slot0, b0, P.keep.data(), nb,
-                                                   P.okey.data(), P.oval.data(), P.tkey.data(),
-                                                   P.tval.data());
+        uint32_t* tkey = scratch.take<uint32_t>(static_cast<size_t>(n_kept));
+        float* tval = scratch.take<float>(static_cast<size_t>(n_kept));
+        pack_pairs_kernel<<<sms * 16, 256, 0, s>>>(slot, a.slot0, b0, kept, nb, okey, oval, tkey,
+                                                   tval);
         cuda_check(cudaGetLastError(), "pack_pairs_kernel");
         steps.mark("pack");
-        emit_columns(ESZ, nl, n_kept, s, P, steps, out, ltp);
+        pieces.push_back(emit_columns(ESZ, nl, n_kept, tkey, tval, list_koff, cols, s, scratch,
+                                      keep, steps, ltp));
+        cols += static_cast<size_t>(pieces.back().n_cols);
+        scratch.release(batch);
         t0 = t1;
     }
+    scratch.release(start);
+    join_columns(ESZ, pieces, s, out);
+    steps.mark("join");
 }
 
 }  // namespace
 
 void summarize_blocks(int esz, const FwdView& f, const BlockSet& blocks, float alpha,
-                      const HostCsr* host, cudaStream_t s, DevColumns& out,
+                      const HostCsr* host, cudaStream_t s, Arena& scratch, DevColumns& out,
                       std::vector<int64_t>& ltp,
                       std::vector<std::pair<std::string, double>>* step_times) {
     Steps steps{step_times, s};
-    if (esz == 4) summarize_typed<4>(f, blocks, alpha, host, s, out, ltp, steps);
-    else if (esz == 2) summarize_typed<2>(f, blocks, alpha, host, s, out, ltp, steps);
-    else summarize_typed<1>(f, blocks, alpha, host, s, out, ltp, steps);
+    if (esz == 4) summarize_typed<4>(f, blocks, alpha, host, s, scratch, out, ltp, steps);
+    else if (esz == 2) summarize_typed<2>(f, blocks, alpha, host, s, scratch, out, ltp, steps);
+    else summarize_typed<1>(f, blocks, alpha, host, s, scratch, out, ltp, steps);
 }
 
 }  // namespace nsp

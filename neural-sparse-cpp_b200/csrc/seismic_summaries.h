@@ -20,10 +20,8 @@ namespace nsp {
 // handed to the device image without a round trip through host memory.
 struct DevColumns {
     DevArray<uint16_t> sterm, sblk;
-    DevArray<int64_t> srun;
+    DevArray<int64_t> srun;  // a boundary per column, and the first
     DevArray<uint8_t> sval;
-    size_t n_cols = 0;     // sterm used; srun holds n_cols + 1 boundaries
-    size_t n_entries = 0;  // sblk used; sval holds n_entries * esz bytes
 };
 
 // Blocks of the lists, as the build's earlier phases leave them.
@@ -36,13 +34,13 @@ struct BlockSet {
     const uint16_t* d_local;  // [n_blocks]: the block's index within its list
 };
 
-// Appends every list's summary columns to `out` and its column prefix to
-// `ltp` (which starts as {0}). `host`: the host rows of an fp32 index, whose
+// Fills `out` with every list's summary columns and appends its column prefix
+// to `ltp` (which starts as {0}). `host`: the host rows of an fp32 index, whose
 // blocks with equal maxima across the alpha cut take the reference's choice
 // (nullptr: value descending, then term ascending, as the codes do).
 // `steps`: time per step, when not null (each step then synchronizes).
 void summarize_blocks(int esz, const FwdView& f, const BlockSet& blocks, float alpha,
-                      const HostCsr* host, cudaStream_t s, DevColumns& out,
+                      const HostCsr* host, cudaStream_t s, Arena& scratch, DevColumns& out,
                       std::vector<int64_t>& ltp,
                       std::vector<std::pair<std::string, double>>* steps);
 
