@@ -380,6 +380,39 @@ NSP_RR void cut_like_reference(uint16_t* heap, int n, int cut, Value value) {
     }
 }
 
+// The same on integer codes below 2^16, with the holder's entries as words
+// code << 16 | position (one load per entry instead of two dependent ones).
+// `heap` has room for `cut` words; it ends as cut_like_reference's order.
+struct WordGreater {
+    NSP_RR bool operator()(uint32_t x, uint32_t y) const { return (x >> 16) > (y >> 16); }
+};
+
+template <typename Code>
+NSP_RR void cut_words_like_reference(uint32_t* heap, int n, int cut, const Code* codes) {
+    const WordGreater less{};
+    int m = 0;
+    for (int i = 0; i < n; ++i) {
+        const uint32_t w = (static_cast<uint32_t>(codes[i]) << 16) | static_cast<uint32_t>(i);
+        if (m >= cut && !less(w, heap[0])) continue;
+        if (m >= cut) {
+            if (m > 1) {
+                const uint32_t v = heap[m - 1];
+                heap[m - 1] = heap[0];
+                heap_sift_down(heap, 0, m - 1, v, less);
+            }
+            --m;
+        }
+        heap_sift_up(heap, m, 0, w, less);
+        ++m;
+    }
+    while (m > 1) {
+        const uint32_t v = heap[m - 1];
+        heap[m - 1] = heap[0];
+        heap_sift_down(heap, 0, m - 1, v, less);
+        --m;
+    }
+}
+
 }  // namespace ranking
 }  // namespace nsp
 

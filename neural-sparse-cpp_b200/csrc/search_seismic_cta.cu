@@ -62,6 +62,7 @@ using detail_search::kFull;
 using detail_search::ValT;
 
 constexpr int kSegCap = 128;    // block segments per batch, one CTA per query
+constexpr int kSortQueue = 64;  // ranges sorted side by side (two per warp at most)
 constexpr int kSegCapMax = 1024;  // the most any launch asks for (a cluster per query)
 
 // A run of consecutive docs of one block inside a batch.
@@ -72,8 +73,20 @@ struct Seg {
     int32_t blk;    // block index within its list
     float bs;       // the block's summary score
     int32_t head;   // 1 when the block starts here (its pruning test applies)
-    int32_t surv;   // 1 when a doc of it may still enter the heap (set after scoring)
+    uint32_t best;  // key of its best member score above the heap minimum at the gather (0: none)
 };
+
+// Order-preserving keys of scores, above 0 (NaN sorts past every number: a
+// NaN score passes every `score <= minimum` rejection, as it does there).
+__device__ __forceinline__ uint32_t score_key(float v) {
+    if (v != v) return 0xffffffffu;
+    const uint32_t b = __float_as_uint(v);
+    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+__device__ __forceinline__ float key_score(uint32_t k) {
+    if (k == 0xffffffffu) return __uint_as_float(0x7fc00000u);
+    return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
+}
 
 struct Ctl {
     int32_t q;
@@ -88,7 +101,7 @@ __host__ __device__ inline size_t a16(size_t x) { return (x + 15) & ~size_t(15);
 
 struct CtaLayout {
     size_t tbl, qv, qterm, qraw, cuts, hs, hid, cdoc, coff, clen, csc, segs, cseg, wsum, cur, uq,
-        total;
+        sq, total;
 };
 
 // Shared-memory layout of one CTA. The four candidate arrays are contiguous
@@ -113,6 +126,7 @@ __host__ __device__ inline CtaLayout cta_layout(int vsize, int tsize, int dim, i
     L.wsum = o;  o += 32 * 4;
     L.cur = o;   o += 64;  // warp 0's Cursor
     L.uq = o;    o += 2 * 32 * 4;  // counting pass: warp 0's per-lane unique docs, row bytes
+    L.sq = o;    o += 2 * kSortQueue * 4 + 16;  // ranges of the first list's sort
     L.total = o;
     return L;
 }
@@ -450,18 +464,238 @@ __device__ void list_summaries(const SeismicLaunch& a, int t, int nb, const uint
     }
 }
 
-// The first list's visiting order: the reference's std::ranges::sort of the
-// block indices by summary score descending (seismic_common.h:105-115),
-// restated in ref_ranking.cuh -- equal scores keep the order the reference's
-// unstable sort leaves. Warp 0 sorts (score, block) pairs in `items`; the
-// other warps wait at the barrier.
-__device__ void sort_blocks(const float* bscore, int nb, ranking::Blk* items, uint16_t* order,
-                            int tid, int warp, int lane) {
-    if (warp == 0) {
-        for (int i = lane; i < nb; i += 32) items[i] = ranking::Blk{__ldcg(bscore + i), i};
+// ------------------------------------------------ the first list's sort --
+// The visiting order of the first list is the reference's std::ranges::sort
+// of the block indices by summary score descending (seismic_common.h:105-115):
+// equal scores keep the order that unstable sort leaves (ref_ranking.cuh).
+// Its partition steps are Hoare's: the k-th element from the left that does
+// not come before the pivot is swapped with the k-th from the right that the
+// pivot does not come before, as long as they have not met. Which elements
+// those are does not depend on the swaps, so a warp finds them with ballots
+// and swaps all pairs at once. Ranges are disjoint, so warps take them side
+// by side, and ranges of at most 16 elements, which the reference leaves to
+// its insertion pass, are stable-sorted by rank. One lane per range took 105
+// us for a lone query's 400 blocks and 180 us for 600 (fp32 100k docs, SQ 3M).
+
+// One partition step of a[f, l), l - f > 16, by a warp; returns the cut.
+// `stops` has room for l entries.
+__device__ int warp_partition(ranking::Blk* a, int f, int l, uint16_t* stops, int lane) {
+    const int x = f + 1, y = f + (l - f) / 2, z = l - 1;
+    const ranking::Blk vx = a[x], vy = a[y], vz = a[z], vf = a[f];
+    int m;
+    if (ranking::before(vx, vy)) {
+        if (ranking::before(vy, vz)) m = y;
+        else m = ranking::before(vx, vz) ? z : x;
+    } else if (ranking::before(vx, vz)) {
+        m = x;
+    } else {
+        m = ranking::before(vy, vz) ? z : y;
+    }
+    const ranking::Blk p = m == x ? vx : (m == y ? vy : vz);
+    __syncwarp();
+    if (lane == 0) {
+        a[f] = p;
+        a[m] = vf;
+    }
+    __syncwarp();
+    // at most K pairs are swapped, so the first K + 1 stops from the left and
+    // K from the right decide
+    const int K = (l - f - 1) / 2;
+    uint16_t* ls = stops + f;
+    uint16_t* rs = ls + K + 1;
+    const unsigned below = (1u << lane) - 1u;
+    int nl = 0, nr = 0;
+    for (int b = f + 1; b < l && nl <= K; b += 32) {
+        const int i = b + lane;
+        const bool st = i < l && !ranking::before(a[i], p);
+        const unsigned w = __ballot_sync(kFull, st);
+        const int at = nl + __popc(w & below);
+        if (st && at <= K) ls[at] = static_cast<uint16_t>(i);
+        nl += __popc(w);
+    }
+    for (int b = l - 1; b >= f && nr < K; b -= 32) {
+        const int i = b - lane;
+        const bool st = i >= f && !ranking::before(p, a[i]);
+        const unsigned w = __ballot_sync(kFull, st);
+        const int at = nr + __popc(w & below);
+        if (st && at < K) rs[at] = static_cast<uint16_t>(i);
+        nr += __popc(w);
+    }
+    nl = min(nl, K + 1);
+    nr = min(nr, K);
+    __syncwarp();
+    int pairs = 0;
+    for (int k0 = 0;; k0 += 32) {
+        const int k = k0 + lane;
+        const bool ok = k < nl && k < nr && ls[k] < rs[k];
+        if (ok) {
+            const int lo = ls[k], hi = rs[k];
+            const ranking::Blk t = a[lo];
+            a[lo] = a[hi];
+            a[hi] = t;
+        }
+        const unsigned w = __ballot_sync(kFull, ok);
+        pairs += __popc(w);
+        if (w != kFull) break;
+    }
+    // the scan from the left ends at its next stop, or at the last element it
+    // swapped to the right
+    int cut = pairs < nl ? ls[pairs] : l;
+    if (pairs > 0) cut = min(cut, static_cast<int>(rs[pairs - 1]));
+    __syncwarp();
+    return cut;
+}
+
+// a[f, l), at most 16 elements, as the insertion pass leaves it.
+__device__ void warp_insertion(ranking::Blk* a, int f, int l, int lane) {
+    const int n = l - f;
+    if (n < 2) return;
+    ranking::Blk v{0.0f, 0};
+    if (lane < n) v = a[f + lane];
+    if (__any_sync(kFull, v.s != v.s)) {  // NaN scores have no rank
+        if (lane == 0) ranking::insertion_range(a, f, l);
         __syncwarp();
-        ranking::warp_sort_blocks_like_reference(items, nb, lane);
-        for (int i = lane; i < nb; i += 32) order[i] = static_cast<uint16_t>(items[i].b);
+        return;
+    }
+    int r = 0;
+    for (int j = 0; j < n; ++j) {
+        const float x = __shfl_sync(kFull, v.s, j);
+        r += (x > v.s || (x == v.s && j < lane)) ? 1 : 0;
+    }
+    __syncwarp();
+    if (lane < n) a[f + r] = v;
+    __syncwarp();
+}
+
+// The introsort loop over a[f, l) with depth budget d by a warp, then the
+// insertion pass. Lane i holds pending range i (their budgets strictly
+// decrease, so at most 2 * 16 wait at once for lists of up to 65,536 blocks).
+__device__ void warp_sort_range(ranking::Blk* a, int f, int l, int d, uint16_t* stops, int lane) {
+    int pf = 0, pl = 0, pd = 0;
+    int sp = 0;
+    for (;;) {
+        while (l - f > ranking::kSortThreshold && d > 0) {
+            --d;
+            const int cut = warp_partition(a, f, l, stops, lane);
+            if (l - cut > ranking::kSortThreshold && sp < 32) {
+                if (lane == sp) {
+                    pf = cut;
+                    pl = l;
+                    pd = d;
+                }
+                ++sp;
+            } else {
+                warp_insertion(a, cut, l, lane);
+            }
+            l = cut;
+        }
+        if (l - f > ranking::kSortThreshold) {  // the depth budget is spent
+            if (lane == 0) ranking::heap_sort_range(a, f, l);
+            __syncwarp();
+        } else {
+            warp_insertion(a, f, l, lane);
+        }
+        if (sp == 0) return;
+        --sp;
+        f = __shfl_sync(kFull, pf, sp);
+        l = __shfl_sync(kFull, pl, sp);
+        d = __shfl_sync(kFull, pd, sp);
+    }
+}
+
+// All threads: (score, block) pairs into `items`, sorted, block indices into
+// order[0..nb). `stops`: scratch of nb entries, which may be `order`.
+__device__ void sort_blocks(const float* bscore, int nb, ranking::Blk* items, uint16_t* stops,
+                            uint16_t* order, uint32_t* queue, int tid, int lane, int warp,
+                            int nwarps) {
+    for (int i = tid; i < nb; i += blockDim.x) items[i] = ranking::Blk{__ldcg(bscore + i), i};
+    // ranges as first | (last << 16); both queues, then their sizes
+    uint32_t* cnt = queue + 2 * kSortQueue;
+    if (tid == 0) {
+        queue[0] = static_cast<uint32_t>(nb - 1) << 16;
+        cnt[0] = 1u;
+        cnt[1] = 0u;
+    }
+    __syncthreads();
+    int n = 1, q = 0, d = 2 * ranking::floor_log2(nb);
+    // level by level until every warp has a range
+    while (n > 0 && n < nwarps && d > 0) {
+        --d;
+        if (warp < n) {
+            const uint32_t r = queue[q * kSortQueue + warp];
+            const int f = static_cast<int>(r & 0xffffu), l = static_cast<int>(r >> 16) + 1;
+            if (l - f > ranking::kSortThreshold) {
+                const int cut = warp_partition(items, f, l, stops, lane);
+                const int fs[2] = {f, cut}, es[2] = {cut, l};
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    if (es[u] - fs[u] > ranking::kSortThreshold) {
+                        if (lane == 0)
+                            queue[(q ^ 1) * kSortQueue + atomicAdd(cnt + (q ^ 1), 1u)] =
+                                static_cast<uint32_t>(fs[u]) |
+                                (static_cast<uint32_t>(es[u] - 1) << 16);
+                    } else {
+                        warp_insertion(items, fs[u], es[u], lane);
+                    }
+                }
+            } else {
+                warp_insertion(items, f, l, lane);
+            }
+        }
+        __syncthreads();
+        q ^= 1;
+        n = static_cast<int>(cnt[q]);
+        if (tid == 0) cnt[q ^ 1] = 0u;
+        __syncthreads();
+    }
+    for (int i = warp; i < n; i += nwarps) {
+        const uint32_t r = queue[q * kSortQueue + i];
+        warp_sort_range(items, static_cast<int>(r & 0xffffu), static_cast<int>(r >> 16) + 1, d,
+                        stops, lane);
+    }
+    __syncthreads();
+    for (int i = tid; i < nb; i += blockDim.x) order[i] = static_cast<uint16_t>(items[i].b);
+    __syncthreads();
+}
+
+// --------------------------------------------------------- the query cut --
+// cuts[0..ncut) = positions of the query's ncut largest weights in the order
+// of the reference's holder (utils/vector_process.h:18-30). Distinct weights
+// come out by value descending, so every thread ranks one; where two of the
+// kept weights are equal (or one is NaN) one thread repeats the holder's
+// steps -- on (code, position) words for codes, which tie constantly, where
+// `room` words hold them. Ranking costs qn loads per thread, so very long
+// queries take the one-thread steps at once (a lone fp32 query's cut of 10
+// from 29 terms: 9 us on one thread; SQ, 12 from 102: 25 us on positions).
+template <typename V>
+__device__ void query_cut(uint16_t* cuts, const V* qraw, int qn, int ncut, uint32_t* words,
+                          int room, int tid) {
+    if constexpr (std::is_same<V, float>::value) {
+        bool tie = qn > 1024;
+        if (!tie)
+            for (int i = tid; i < qn; i += blockDim.x) {
+                const float v = qraw[i];
+                int r = 0;
+                bool eq = v != v;
+                for (int j = 0; j < qn; ++j) {
+                    const float x = qraw[j];
+                    r += x > v ? 1 : 0;
+                    eq |= (x == v && j != i) || x != x;
+                }
+                if (r < ncut) {
+                    tie |= eq;
+                    if (!eq) cuts[r] = static_cast<uint16_t>(i);
+                }
+            }
+        if (!__syncthreads_or(tie)) return;
+        if (tid == 0) ranking::cut_like_reference(cuts, qn, ncut, QueryWeight<V>{qraw});
+    } else {
+        if (ncut > room) {
+            if (tid == 0) ranking::cut_like_reference(cuts, qn, ncut, QueryWeight<V>{qraw});
+        } else if (tid == 0) {
+            ranking::cut_words_like_reference(words, qn, ncut, qraw);
+            for (int i = 0; i < ncut; ++i) cuts[i] = static_cast<uint16_t>(words[i]);
+        }
     }
     __syncthreads();
 }
@@ -500,7 +734,7 @@ __device__ int gather(const SeismicLaunch& a, Cursor& c, bool first, int64_t lb0
             g.blk = c.split_blk;
             g.bs = c.split_bs;
             g.head = 0;
-            g.surv = 0;
+            g.best = 0u;
             segs[0] = g;
         }
         nseg = 1;
@@ -558,7 +792,7 @@ __device__ int gather(const SeismicLaunch& a, Cursor& c, bool first, int64_t lb0
             g.blk = blk;
             g.bs = bs;
             g.head = 1;
-            g.surv = 0;
+            g.best = 0u;
             segs[nseg + r] = g;
         }
         int taken_docs = 0;
@@ -803,8 +1037,8 @@ __global__ void __launch_bounds__(1024, 1) seismic_cta_kernel(SeismicLaunch a) {
             for (int i = tid; i < qn; i += blockDim.x) cuts[i] = qterm[i];
         } else {
             ncut = a.cut;
-            if (tid == 0) ranking::cut_like_reference(cuts, qn, ncut, QueryWeight<V>{qraw});
-            __syncthreads();
+            query_cut<V>(cuts, qraw, qn, ncut, reinterpret_cast<uint32_t*>(smem + L.cdoc),
+                         static_cast<int>((L.wsum - L.cdoc) / 4), tid);
             for (int i = tid; i < ncut; i += blockDim.x) cuts[i] = qterm[cuts[i]];
         }
         __syncthreads();
@@ -850,15 +1084,20 @@ __global__ void __launch_bounds__(1024, 1) seismic_cta_kernel(SeismicLaunch a) {
                 // list's blocks that can still pass, in block order
                 int nbv = nb;
                 if (first) {
-                    int p2 = 1;
-                    while (p2 < nb) p2 <<= 1;
+                    // in the batch arrays' place where they are large enough
+                    const size_t room = L.wsum - L.cdoc;
+                    const size_t pairs = static_cast<size_t>(nb) * sizeof(ranking::Blk);
                     ranking::Blk* items = reinterpret_cast<ranking::Blk*>(
-                        p2 <= 2 * batch ? reinterpret_cast<unsigned long long*>(cdoc) : keys_g);
+                        pairs <= room ? reinterpret_cast<unsigned long long*>(cdoc) : keys_g);
                     if (items == nullptr) {  // the host sizes sortkeys; never taken
                         if (tid == 0) atomicExch(a.err, 2);
                         break;
                     }
-                    sort_blocks(bscore, nb, items, order, tid, warp, lane);
+                    uint16_t* stops = pairs + static_cast<size_t>(nb) * 2 <= room
+                                          ? reinterpret_cast<uint16_t*>(smem + L.cdoc + pairs)
+                                          : order;
+                    sort_blocks(bscore, nb, items, stops, order,
+                                reinterpret_cast<uint32_t*>(smem + L.sq), tid, lane, warp, nwarps);
                 } else {
                     const int nh = ctl->nheap;
                     nbv = passing_blocks(bscore, nb, nh == a.k, nh == a.k ? hs[0] : 0.0f,
@@ -936,7 +1175,7 @@ __global__ void __launch_bounds__(1024, 1) seismic_cta_kernel(SeismicLaunch a) {
                     // (a) All threads: a doc can still enter the heap only if
                     // it is a member scoring above the heap minimum as it
                     // stood when the batch was gathered (the minimum only
-                    // grows); segments holding such docs are flagged.
+                    // grows); segments take the best score of such docs.
                     {
                         const int nh = ctl->nheap;
                         const float hmin0 = nh == a.k ? hs[0] : 0.0f;
@@ -944,8 +1183,8 @@ __global__ void __launch_bounds__(1024, 1) seismic_cta_kernel(SeismicLaunch a) {
                             if (cdoc[i] >= 0) {
                                 ++docs_scored;
                                 row_bytes += 8 + static_cast<int32_t>(clen[i]) * (2 + vsz);
-                                // a flag: every writer stores the same 1
-                                if (nh < a.k || !(csc[i] <= hmin0)) segs[cseg[i]].surv = 1;
+                                if (nh < a.k || !(csc[i] <= hmin0))
+                                    atomicMax(&segs[cseg[i]].best, score_key(csc[i]));
                             }
                         }
                         __syncthreads();
@@ -958,11 +1197,11 @@ __global__ void __launch_bounds__(1024, 1) seismic_cta_kernel(SeismicLaunch a) {
                     // so all its tests see one minimum and one ballot settles
                     // up to 32 of them; a segment with survivors offers those.
                     if (warp == 0) {
-                        // the work counters give back a dropped segment's docs
-                        auto give_back = [&](int t) {
-                            const Seg g = segs[t];
-                            for (int j = lane; j < g.cnt; j += 32) {
-                                const int i = g.cand0 + j;
+                        // the work counters give back dropped segments' docs
+                        // (segment after segment, their candidates are
+                        // contiguous: a lone query drops hundreds at once)
+                        auto give_back = [&](int c0, int c1) {
+                            for (int i = c0 + lane; i < c1; i += 32) {
                                 if (cdoc[i] >= 0) {
                                     --docs_scored;
                                     row_bytes -= 8 + static_cast<int32_t>(clen[i]) * (2 + vsz);
@@ -987,98 +1226,113 @@ __global__ void __launch_bounds__(1024, 1) seismic_cta_kernel(SeismicLaunch a) {
                             }
                         };
                         auto end_first_list = [&](int from) {
-                            for (int t = from; t < nseg; ++t) give_back(t);
+                            give_back(segs[from].cand0, total);
                             cur.dead = true;
                             cur.split = false;
                         };
-                        int s = 0;
                         bool ended = false;
-                        while (s < nseg && !ended) {
-                            const int sl = s + lane;
-                            const bool valid = sl < nseg;
-                            int head = 0, cnt = 0, surv = 0;
+                        for (int s0 = 0; s0 < nseg && !ended; s0 += 32) {
+                            const bool valid = s0 + lane < nseg;
+                            int head = 0, cnt = 0, cand0 = 0;
+                            uint32_t best = 0u;
                             float bs = 0.0f;
                             if (valid) {
-                                const Seg g = segs[sl];
+                                const Seg g = segs[s0 + lane];
                                 head = g.head;
                                 cnt = g.cnt;
-                                surv = g.surv;
+                                cand0 = g.cand0;
+                                best = g.best;
                                 bs = g.bs;
                             }
-                            const int w = __popc(__ballot_sync(kFull, valid));
-                            const unsigned sm = __ballot_sync(kFull, valid && surv > 0);
-                            const int S = sm ? __ffs(sm) - 1 : w;  // first that may change the heap
-                            const bool full = n == a.k;
-                            const float hmin = full ? hs[0] : 0.0f;
-                            const bool fail =
-                                lane < S && head && full && __fmul_rn(bs, a.heap_factor) < hmin;
-                            const unsigned fm = __ballot_sync(kFull, fail);
-                            // the first list ends at its first failing block
-                            const int upto = (first && fm) ? __ffs(fm) - 1 : S;
-                            const bool taken = lane < upto && !fail;
-                            blocks_visited += __popc(__ballot_sync(kFull, taken && head));
-                            bytes += 16u * __popc(__ballot_sync(kFull, taken && head)) +
-                                     4u * __reduce_add_sync(kFull, taken ? cnt : 0);
-                            if (a.visit != nullptr) {
-                                unsigned tm = __ballot_sync(kFull, taken);
-                                while (tm) {
-                                    const int t = __ffs(tm) - 1;
-                                    tm &= tm - 1;
-                                    count_visits(s + t);
+                            const int w = min(32, nseg - s0);
+                            int pos = 0;
+                            while (pos < w) {
+                                const bool full = n == a.k;
+                                const float hmin = full ? hs[0] : 0.0f;
+                                // the first segment that may change the heap
+                                const unsigned sm =
+                                    __ballot_sync(kFull, lane >= pos && best != 0u &&
+                                                             (!full || !(key_score(best) <= hmin)));
+                                const int S = sm ? __ffs(sm) - 1 : w;
+                                const bool fails = head && full &&
+                                                   __fmul_rn(bs, a.heap_factor) < hmin;
+                                const bool run = lane >= pos && lane < S;
+                                const unsigned fm = __ballot_sync(kFull, run && fails);
+                                // the first list ends at its first failing block
+                                const int upto = (first && fm) ? __ffs(fm) - 1 : S;
+                                const bool taken = run && lane < upto && !fails;
+                                const int heads = __popc(__ballot_sync(kFull, taken && head));
+                                blocks_visited += heads;
+                                bytes += 16u * heads +
+                                         4u * __reduce_add_sync(kFull, taken ? cnt : 0);
+                                if (a.visit != nullptr) {
+                                    unsigned tm = __ballot_sync(kFull, taken);
+                                    while (tm) {
+                                        const int t = __ffs(tm) - 1;
+                                        tm &= tm - 1;
+                                        count_visits(s0 + t);
+                                    }
                                 }
-                            }
-                            unsigned dm = __ballot_sync(kFull, lane < upto && fail);
-                            while (dm) {  // later lists skip a failing block
-                                const int t = __ffs(dm) - 1;
-                                dm &= dm - 1;
-                                give_back(s + t);
-                                if (s + t == nseg - 1) cur.split = false;
-                            }
-                            if (first && fm) {
-                                end_first_list(s + upto);
-                                ended = true;
-                                break;
-                            }
-                            s += upto;
-                            if (upto == w) continue;
-                            // segment s holds survivors: its test, then its offers
-                            const Seg g = segs[s];
-                            if (g.head && n == a.k &&
-                                __fmul_rn(g.bs, a.heap_factor) < hs[0]) {
-                                if (first) {
-                                    end_first_list(s);
+                                if (first && fm) {
+                                    end_first_list(s0 + upto);
                                     ended = true;
                                     break;
                                 }
-                                give_back(s);
-                                if (s == nseg - 1) cur.split = false;
-                            } else {
-                                if (g.head) {
-                                    ++blocks_visited;
-                                    bytes += 16;
+                                unsigned dm = fm;
+                                while (dm) {  // later lists skip failing blocks, run by run
+                                    const int t = __ffs(dm) - 1;
+                                    const unsigned rest = ~(dm >> t);
+                                    const int len = rest ? __ffs(rest) - 1 : 32;
+                                    const int last = min(t + len, 32) - 1;
+                                    dm &= last == 31 ? 0u : ~0u << (last + 1);
+                                    give_back(__shfl_sync(kFull, cand0, t),
+                                              __shfl_sync(kFull, cand0 + cnt, last));
+                                    if (s0 + last == nseg - 1) cur.split = false;
                                 }
-                                bytes += 4u * static_cast<uint32_t>(g.cnt);
-                                count_visits(s);
-                                for (int b = 0; b < g.cnt; b += 32) {
-                                    const int j = b + lane;
-                                    float sc = 0.0f;
-                                    int32_t d = -1;
-                                    if (j < g.cnt) {
-                                        d = cdoc[g.cand0 + j];
-                                        sc = csc[g.cand0 + j];
+                                pos = upto;
+                                if (pos == w) break;
+                                // its test, then its offers
+                                if (__shfl_sync(kFull, fails ? 1 : 0, pos)) {
+                                    if (first) {
+                                        end_first_list(s0 + pos);
+                                        ended = true;
+                                        break;
                                     }
-                                    unsigned m = __ballot_sync(
-                                        kFull, d >= 0 && (n < a.k || !(sc <= hs[0])));
-                                    while (m) {
-                                        const int src = __ffs(m) - 1;
-                                        m &= m - 1;
-                                        const float S2 = __shfl_sync(kFull, sc, src);
-                                        const int32_t D2 = __shfl_sync(kFull, d, src);
-                                        heap_offer(S2, D2, hs, hid, n, a.k, lane);
+                                    const int c0 = __shfl_sync(kFull, cand0, pos);
+                                    give_back(c0, c0 + __shfl_sync(kFull, cnt, pos));
+                                    if (s0 + pos == nseg - 1) cur.split = false;
+                                } else {
+                                    const int gcnt = __shfl_sync(kFull, cnt, pos);
+                                    const int g0 = __shfl_sync(kFull, cand0, pos);
+                                    if (__shfl_sync(kFull, head, pos)) {
+                                        ++blocks_visited;
+                                        bytes += 16;
+                                    }
+                                    bytes += 4u * static_cast<uint32_t>(gcnt);
+                                    count_visits(s0 + pos);
+                                    for (int b = 0; b < gcnt; b += 32) {
+                                        const int j = b + lane;
+                                        float sc = 0.0f;
+                                        int32_t d = -1;
+                                        if (j < gcnt) {
+                                            d = cdoc[g0 + j];
+                                            sc = csc[g0 + j];
+                                        }
+                                        unsigned m = __ballot_sync(
+                                            kFull, d >= 0 && (n < a.k || !(sc <= hs[0])));
+                                        while (m) {
+                                            const int src = __ffs(m) - 1;
+                                            m &= m - 1;
+                                            const float S2 = __shfl_sync(kFull, sc, src);
+                                            const int32_t D2 = __shfl_sync(kFull, d, src);
+                                            heap_offer(S2, D2, hs, hid, n, a.k, lane);
+                                            // the others against the new minimum
+                                            m &= __ballot_sync(kFull, n < a.k || !(sc <= hs[0]));
+                                        }
                                     }
                                 }
+                                ++pos;
                             }
-                            ++s;
                         }
                     }
                 }
