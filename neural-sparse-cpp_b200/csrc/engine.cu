@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 #include <numeric>
@@ -1029,7 +1030,13 @@ void exact_search(const ForwardDevice& fwd, const PostingsDevice* post, const Qu
     if (taat) {
         // term at a time: candidates per (query, doc chunk), no per-lane lists
         a.post = post->view();
-        const size_t cands = static_cast<size_t>(q.n) * a.post.n_chunks * k;
+        // (non-finite query values can give NaN scores, whose order depends
+        // on the parts: they keep whole chunks)
+        bool finite = true;
+        for (int64_t i = q.ip[0]; i < q.ip[q.n]; ++i) finite &= std::isfinite(q.vv[i]);
+        a.dense = finite && a.post.n_dense > 0;
+        a.splits = finite ? exact_taat_splits(q.n, a.post.n_chunks, a.post.chunk_docs, sms) : 1;
+        const size_t cands = static_cast<size_t>(q.n) * a.post.n_chunks * a.splits * k;
         a.cand_d = static_cast<float*>(ws.dev(Workspace::kCandD, cands * sizeof(float)));
         a.cand_l = static_cast<int32_t*>(ws.dev(Workspace::kCandL, cands * sizeof(int32_t)));
     } else {

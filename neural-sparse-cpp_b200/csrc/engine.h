@@ -212,9 +212,12 @@ private:
     bool usable_ = false;
     int32_t n_chunks_ = 0;
     int32_t chunk_docs_ = 0;
+    int32_t n_dense_ = 0;
     DevArray<int32_t> doc_;
     DevArray<float> val_;
     DevArray<int32_t> chunk_at_;
+    DevArray<int16_t> dense_of_;
+    DevArray<float> dense_;
 };
 
 // SEISMIC lists flattened over terms, in host memory (the reference's

@@ -166,11 +166,19 @@ struct PostingsView {
     const int32_t* doc;
     const float* val;
     const int32_t* chunk_at;    // [dim][n_chunks + 1]
+    // Terms held by at least kDenseShare of the docs also as dense rows:
+    // dense[(c * n_dense + j) * chunk_docs + d] is dense term j's value in doc
+    // d of chunk c, 0 where the doc lacks it; dense_of[term] = j or -1.
+    int32_t n_dense;
+    const int16_t* dense_of;
+    const float* dense;
 };
 
 struct ExactLaunch {
     FwdView fwd;
     PostingsView post;          // term-at-a-time path (launch_exact_taat)
+    int splits;                 // CTAs per doc chunk on that path (a divisor of its docs)
+    bool dense;                 // frequent terms from their dense rows (finite weights)
     QueryView q;
     int k;
     int mode;                   // 0 brutal (all docs), 1 inverted (score > 0)
@@ -228,9 +236,11 @@ size_t exact_smem(int dim_words, int qcap_smem);  // qcap_smem 0: values in glob
 cudaError_t launch_exact(const ExactLaunch& a, int tiles, cudaStream_t s);
 
 // Term-at-a-time exact search (search_exact_taat.cu): one CTA per (query, doc
-// chunk of a.post), k <= kTaatMaxK; candidates per chunk in a.cand_d/l
+// chunk of a.post), k <= kTaatMaxK; candidates per (query, chunk part) in a.cand_d/l
 // [n_q][n_chunks][k], then the tile path's merge.
 constexpr int kTaatMaxK = 128;
+// CTAs per doc chunk for a launch of n_queries.
+int exact_taat_splits(int n_queries, int n_chunks, int chunk_docs, int sms);
 int exact_taat_chunk_docs();  // docs per chunk that keep 4 CTAs per SM
 cudaError_t launch_exact_taat(const ExactLaunch& a, cudaStream_t s);
 
