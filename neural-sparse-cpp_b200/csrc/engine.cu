@@ -562,6 +562,8 @@ int auto_cluster(int n_queries) {
     const int sms = device_sm_count();
     int c = 1;
     while (c < 8 && static_cast<long long>(std::max(n_queries, 1)) * (c * 2) <= sms) c *= 2;
+    // 16 CTAs fill a GPC, so only a few such clusters run at once
+    if (c == 8 && static_cast<long long>(std::max(n_queries, 1)) * 32 <= sms) c = 16;
     return c;
 }
 
@@ -598,9 +600,9 @@ SeismicPlan plan_seismic_cta(int kind, int dim, int qcap, int k, int n_queries,
         while (batch > 32 && seismic_cta_smem(kind, dim, qcap, k, batch, seg_cap) > limit)
             batch >>= 1;
         p.smem_cta = seismic_cta_smem(kind, dim, qcap, k, batch, seg_cap);
-        // a cluster's larger segment table must not cost the engine's own
-        // choice a query it could run on one CTA
-        if (p.smem_cta <= limit || args.cluster > 0 || cl == 1) break;
+        // a cluster's larger segment table (and its kernel's static shared
+        // memory, below 2 KB) must not refuse a query that one CTA can run
+        if (cl == 1 || p.smem_cta + 2048 <= limit) break;
         cl = 1;
     }
     if (p.smem_cta > limit)

@@ -145,6 +145,8 @@ public:
     cudaStream_t stream() const { return stream_; }
     void* dev(int s, size_t bytes) override;
     void* pinned(Slot s, size_t bytes);
+    // The two events that time a search's kernels on this thread's stream.
+    cudaEvent_t event(int i);
     ~Workspace();
 
 private:
@@ -155,6 +157,7 @@ private:
     size_t dcap_[kNumSlots] = {};
     void* hptr_[kNumSlots] = {};
     size_t hcap_[kNumSlots] = {};
+    cudaEvent_t event_[2] = {};
 };
 
 // Host CSR in the reference's SparseVectors layout (sparse_vectors.h:23-111):

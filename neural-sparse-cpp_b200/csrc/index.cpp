@@ -388,10 +388,11 @@ void apply_tuned(const SeismicState& st, nsp::SeismicSearchArgs& a, int64_t n_qu
     a.variant = st.tuned.variant;
     if (a.cluster == 0 && st.tuned.split > 0) {
         // the split measured fastest for a lone query, where the engine's
-        // rule would give a launch this small a cluster at all
+        // rule would give a launch this small a cluster at all (the largest
+        // split measured leaves the rule its own choice)
         const int rule = nsp::auto_cluster(
             a.plain ? 1 : static_cast<int>(std::min<int64_t>(n_queries, 1 << 30)));
-        a.cluster = std::min(rule, st.tuned.split);
+        a.cluster = st.tuned.split < 8 ? std::min(rule, st.tuned.split) : rule;
     }
     if (a.plain || n_queries <= 2 * static_cast<int64_t>(nsp::device_sm_count())) return;
     if (a.batch_docs == 0) a.batch_docs = st.tuned.batch_docs;

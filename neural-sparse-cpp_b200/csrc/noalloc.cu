@@ -179,9 +179,11 @@ extern "C" nsp_status_t nsp_index_search_device_noalloc(
             return static_cast<long long>((avail - nd.fixed - slack) / nd.per_cta);
         };
         long long room = fits(need);
-        if (room < need.cluster && need.cluster > 1 && a.cluster <= 0) {
-            // the engine's cluster does not fit: one CTA per query
-            a.cluster = 1;
+        const bool engines_choice = a.cluster <= 0;
+        while (room < need.cluster && need.cluster > 1 && engines_choice) {
+            // the engine's cluster does not fit: smaller ones (past 8 CTAs),
+            // then one CTA per query
+            a.cluster = need.cluster > 8 ? 8 : 1;
             need = nsp::seismic_scratch_need(st->vectors.dev, st->lists_dev, n, max_row_nnz, a);
             room = fits(need);
         }

@@ -231,6 +231,11 @@ int seismic_cta_max_blocks_per_sm(int val_kind, int qcap, int group_lanes, int w
                                   size_t smem);
 cudaError_t launch_seismic_cta(int val_kind, const SeismicLaunch& a, int warps, int blocks,
                                cudaStream_t s);
+// A cluster of a.cluster CTAs per query (search_seismic_cluster.cu); `placed`:
+// whether the device can place one (nothing is launched otherwise).
+cudaError_t launch_seismic_cluster(int val_kind, const SeismicLaunch& a, int warps, int blocks,
+                                   size_t smem, bool& placed, cudaStream_t s);
+
 
 size_t exact_smem(int dim_words, int qcap_smem);  // qcap_smem 0: values in global
 cudaError_t launch_exact(const ExactLaunch& a, int tiles, cudaStream_t s);

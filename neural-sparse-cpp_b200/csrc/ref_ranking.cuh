@@ -340,6 +340,107 @@ NSP_RR void topk_drain_descending(TopK h, int n, float* out_s, int32_t* out_id) 
     }
 }
 
+#if defined(__CUDACC__)
+// The holder with its entries in a warp's registers (lane i holds entry i, k
+// <= 32, no NaN scores): the same entries in the same places as topk_add
+// leaves, found by all lanes at once. A pop moves entries up along the path
+// of preferred children as far as they are not above the moved last entry
+// (along the path scores do not decrease), a push moves ancestors above the
+// new entry down. All lanes call.
+__device__ __forceinline__ void warp_heap_pop(float& s, int32_t& id, int& n, int lane) {
+    const unsigned all = 0xffffffffu;
+    const int len = n - 1;
+    if (len > 0) {
+        const float vs = __shfl_sync(all, s, len);
+        const int32_t vi = __shfl_sync(all, id, len);
+        const int l = 2 * lane + 1, r = 2 * lane + 2;
+        const float sl = __shfl_sync(all, s, l & 31), sr = __shfl_sync(all, s, r & 31);
+        int child = -1;
+        if (lane < (len - 1) / 2) child = sr > sl ? l : r;
+        else if ((len & 1) == 0 && lane == (len - 2) / 2) child = l;
+        const float cs = __shfl_sync(all, s, child & 31);
+        const int32_t ci = __shfl_sync(all, id, child & 31);
+        unsigned path = 0u;
+        for (int cur = 0; cur >= 0;) {
+            path |= 1u << cur;
+            cur = __shfl_sync(all, child, cur);
+        }
+        if ((path >> lane) & 1u) {
+            const bool stays = child < 0 || cs > vs;  // the child does not move here
+            if (!stays) {
+                s = cs;
+                id = ci;
+            } else if (lane == 0 || !(s > vs)) {
+                s = vs;
+                id = vi;
+            }
+        }
+    }
+    n = len;
+}
+
+__device__ __forceinline__ void warp_heap_push(float& s, int32_t& id, int& n, float ns, int32_t ni,
+                                               int lane) {
+    const unsigned all = 0xffffffffu;
+    unsigned chain = 1u << n;
+    for (int x = n; x > 0;) {
+        x = (x - 1) / 2;
+        chain |= 1u << x;
+    }
+    const int parent = lane > 0 ? (lane - 1) / 2 : 0;
+    const float ps = __shfl_sync(all, s, parent);
+    const int32_t pi = __shfl_sync(all, id, parent);
+    if ((chain >> lane) & 1u) {
+        if (lane > 0 && ps > ns) {
+            s = ps;
+            id = pi;
+        } else if (lane == n || s > ns) {
+            s = ns;
+            id = ni;
+        }
+    }
+    ++n;
+}
+
+// TopKHolder::add of a score that is not rejected.
+__device__ __forceinline__ void warp_heap_add(float& s, int32_t& id, int& n, int k, float ns,
+                                              int32_t ni, int lane) {
+    if (n >= k) warp_heap_pop(s, id, n, lane);
+    warp_heap_push(s, id, n, ns, ni, lane);
+}
+
+// cut_like_reference by a warp for cut <= 32 and weights that are not NaN
+// (`value(i)` of position i): cuts[0..cut) in the holder's order.
+template <typename Value>
+__device__ void warp_cut_like_reference(uint16_t* cuts, int n, int cut, Value value, int lane) {
+    const unsigned all = 0xffffffffu;
+    float s = 0.0f;
+    int32_t id = 0;
+    int m = 0;
+    for (int i0 = 0; i0 < n; i0 += 32) {
+        const float v = i0 + lane < n ? value(static_cast<uint16_t>(i0 + lane)) : 0.0f;
+        unsigned in = __ballot_sync(all, i0 + lane < n);
+        while (in) {
+            // the next position the holder does not reject
+            const float top = __shfl_sync(all, s, 0);
+            in &= __ballot_sync(all, m < cut || !(v <= top));
+            if (in == 0u) break;
+            const int src = __ffs(in) - 1;
+            in &= in - 1;
+            warp_heap_add(s, id, m, cut, __shfl_sync(all, v, src), i0 + src, lane);
+        }
+    }
+    int32_t out = 0;
+    while (m > 0) {
+        const int32_t top = __shfl_sync(all, id, 0);
+        if (lane == m - 1) out = top;
+        warp_heap_pop(s, id, m, lane);
+    }
+    if (lane < cut) cuts[lane] = static_cast<uint16_t>(out);
+    __syncwarp();
+}
+#endif
+
 // ---- the query cut ----------------------------------------------------
 
 // top_k_tokens (utils/vector_process.h:18-30) when cut < n: a TopKHolder of
