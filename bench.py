@@ -161,12 +161,12 @@ def counting_pass(nsparse, idx, q, cut, hf, args, L, D):
 
 def claim_order_launches(n_queries, device=None):
     """1 when a batched search of n_queries runs the engine's claim-order
-    kernel before the search kernel (four or more queries per CTA; the
+    kernel before the search kernel (more queries than CTAs; the
     one-CTA-per-query kernel keeps four 8-warp CTAs per SM), else 0."""
     import torch
     dev = torch.cuda.current_device() if device is None else device
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
-    return 1 if n_queries >= 4 * min(n_queries, 4 * sms) else 0
+    return 1 if n_queries > 4 * sms else 0
 
 
 def replica_throughput(total_ms, e2e_s, n_queries, steps, e2e_steps, world, device=None):

@@ -74,6 +74,15 @@ void* Arena::bytes(size_t n) {
     return p;
 }
 
+static int max_smem_per_sm() {
+    int dev = 0;
+    cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+    int v = 0;
+    cuda_check(cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev),
+               "cudaDeviceGetAttribute");
+    return v;
+}
+
 // ------------------------------------------------------------ workspace --
 
 Workspace::Workspace() {
@@ -571,23 +580,23 @@ namespace {
 
 // Variants 2-5 (one CTA per query). Warps per CTA: 8 when the batch has
 // queries enough to give every SM four CTAs; fewer queries get bigger CTAs
-// (16 or 32 warps, up to a whole SM per query), which shortens each query's
-// sequence of candidate batches -- the latency of small batches and of the
-// one-query-per-launch path -- and, below half a query per SM, a cluster of
-// 2-8 such CTAs per query (auto_cluster). Candidate docs per batch: 64 per
+// (10, 16 or 32 warps, up to a whole SM per query), which shortens each
+// query's sequence of candidate batches -- the latency of small batches and of
+// the one-query-per-launch path -- and, below half a query per SM, a cluster
+// of 2-16 such CTAs per query (auto_cluster). Candidate docs per batch: 64 per
 // warp and CTA unless asked otherwise; the batch shrinks if shared memory is
 // short.
 SeismicPlan plan_seismic_cta(int kind, int dim, int qcap, int k, int n_queries,
-                             const SeismicSearchArgs& args, bool single) {
+                             const SeismicSearchArgs& args, bool single, bool filtered) {
     SeismicPlan p{};
     p.variant = args.variant;
     int warps = args.warps_per_block;
     if (warps <= 0) {
         const int sms = device_sm_count();
         const int per = single ? 1 : std::max(n_queries, 1);
-        warps = 8;
-        if (per * 2 <= sms) warps = 32;
-        else if (per <= 2 * sms) warps = 16;
+        // CTAs per SM that hold all queries at once, up to four
+        const int ctas = std::min(4, std::max(1, (per + sms - 1) / sms));
+        warps = 32 / ctas;
     }
     warps = std::min(std::max(warps, 1), 32);
     const size_t limit = static_cast<size_t>(max_smem_optin());
@@ -596,6 +605,15 @@ SeismicPlan plan_seismic_cta(int kind, int dim, int qcap, int k, int n_queries,
     for (;;) {
         seg_cap = seismic_cta_seg_cap(cl);
         batch = args.batch_docs > 0 ? args.batch_docs : 64 * warps * cl;
+        if (filtered && args.batch_docs <= 0 && cl == 1 && warps >= 8) {
+            // a selector's members are all that is scored of a batch: up to
+            // four times as many candidates while as many CTAs stay resident
+            // (333 fp32 queries over a tenth of 1M docs, k = 100: 2.16 -> 1.41
+            // ms, with the members alone kept and 10 warps per CTA instead of 8)
+            const size_t share = static_cast<size_t>(max_smem_per_sm()) / (32 / warps) - 1024;
+            for (int wide = 256 * warps; wide > batch; wide -= 64)
+                if (seismic_cta_smem(kind, dim, qcap, k, wide, seg_cap) <= share) batch = wide;
+        }
         batch = std::min(std::max((batch + 31) & ~31, 32), 8192);
         while (batch > 32 && seismic_cta_smem(kind, dim, qcap, k, batch, seg_cap) > limit)
             batch >>= 1;
@@ -657,9 +675,6 @@ SeismicPlan plan_seismic(int kind, int words, int qcap, int k, int n_queries,
 // The engine's choice of kernel: one CTA per query with four lanes per doc
 // (variant 4) measured fastest at 1M docs (2.9x variant 0).
 constexpr int kDefaultVariant = 4;
-// Batched launches with at least this many queries per CTA claim them longest
-// row first.
-constexpr int kOrderedClaimsPerCta = 4;
 
 }  // namespace
 
@@ -723,7 +738,8 @@ void run_seismic(const ForwardDevice& fwd, const SeismicDevice& ix, int32_t n,
             pa.cluster = 1;
             pa.max_ctas = device_sm_count();
         }
-        const SeismicPlan p = plan_seismic_cta(kind, a.fwd.dim, a.qcap, a.k, n, pa, args.plain);
+        const SeismicPlan p = plan_seismic_cta(kind, a.fwd.dim, a.qcap, a.k, n, pa, args.plain,
+                                               d_sel != nullptr);
         if (args.count_unique) {
             const size_t stamps = static_cast<size_t>(p.blocks) *
                                   static_cast<size_t>(std::max(a.fwd.n_docs, 1));
@@ -757,11 +773,12 @@ void run_seismic(const ForwardDevice& fwd, const SeismicDevice& ix, int32_t n,
             a.work_counter = static_cast<int32_t*>(ws.dev(Workspace::kCounter, sizeof(int32_t)));
             cuda_check(cudaMemsetAsync(a.work_counter, 0, sizeof(int32_t), s), "memset");
             a.first_query = 0;
-            // several queries per CTA: the longest rows are claimed first, so
+            // more queries than CTAs: the longest rows are claimed first, so
             // the launch does not end on a long query claimed last (16,384
-            // SQ queries at 8.8M docs: -1.0%; by a cost estimate from the
-            // cut lists' lengths: -1.1%)
-            if (n >= kOrderedClaimsPerCta * p.blocks) {
+            // SQ queries at 8.8M docs: -1.0%, by a cost estimate from the
+            // cut lists' lengths -1.1%; 1,001 16-bit queries on 592 CTAs, the
+            // last ones' tail being half of the launch: -5.5%)
+            if (n > p.blocks) {
                 auto* ord = static_cast<int32_t*>(
                     ws.dev(Workspace::kQOrder, static_cast<size_t>(n) * sizeof(int32_t)));
                 cuda_check(launch_order_by_length(d_indptr, n, ord, s), "claim order launch");
@@ -857,7 +874,8 @@ SeismicScratchNeed seismic_scratch_need(const ForwardDevice& fwd, const SeismicD
     need.fixed = kStatCount * sizeof(unsigned long long) + 2 * sizeof(int32_t);
     if (args.variant >= 2) need.fixed += static_cast<size_t>(n) * sizeof(int32_t);
     if (args.variant >= 2) {
-        const SeismicPlan p = plan_seismic_cta(kind, fwd.view().dim, qcap, args.k, n, args, false);
+        const SeismicPlan p = plan_seismic_cta(kind, fwd.view().dim, qcap, args.k, n, args, false,
+                                               false);
         int p2 = 1;
         while (p2 < maxb) p2 <<= 1;
         need.per_cta = static_cast<size_t>(p.wpb) * maxb * sizeof(float) +
@@ -901,12 +919,12 @@ void reserve_seismic_scratch(const ForwardDevice& fwd, const SeismicDevice& ix, 
     ws.dev(Workspace::kCounter, sizeof(int32_t));
     if (args.variant < 2) return;
     const SeismicPlan p = plan_seismic_cta(val_kind_of(args.qbits), fwd.view().dim,
-                                           std::max(max_nnz, 1), args.k, n, args, args.plain);
+                                           std::max(max_nnz, 1), args.k, n, args, args.plain, false);
     const int maxb = std::max(ix.max_blocks(), 1);
     const size_t order_stride = static_cast<size_t>((maxb + 7) & ~7);
     ws.dev(Workspace::kBScore, static_cast<size_t>(p.blocks) * p.wpb * maxb * sizeof(float));
     ws.dev(Workspace::kOrder, static_cast<size_t>(p.blocks) * order_stride * sizeof(uint16_t));
-    if (!args.plain && n >= kOrderedClaimsPerCta * p.blocks)
+    if (!args.plain && n > p.blocks)
         ws.dev(Workspace::kQOrder, static_cast<size_t>(n) * sizeof(int32_t));
     int p2 = 1;
     while (p2 < maxb) p2 <<= 1;

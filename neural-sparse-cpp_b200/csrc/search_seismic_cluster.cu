@@ -234,7 +234,7 @@ __device__ int gather_cta(const SeismicLaunch& a, Shared& sh, bool first, const 
         split = take < c.split_left;
         __syncthreads();
         if (tid == 0) {
-            segs[0] = Seg{d0, take, 0, bs, 0, 0u, 0};
+            segs[0] = Seg{d0, take, 0, bs, 0, 0u, take};
             c.split_d = d0 + take;
             c.split_left -= take;
             c.split = split;
@@ -281,7 +281,7 @@ __device__ int gather_cta(const SeismicLaunch& a, Shared& sh, bool first, const 
         const int nt = __syncthreads_count(take);  // a prefix of the candidates
         if (take) {
             const int cnt = min(sz, room - excl);
-            segs[nseg + r] = Seg{d0, cnt, total + excl, bs, 1, 0u, 0};
+            segs[nseg + r] = Seg{d0, cnt, total + excl, bs, 1, 0u, cnt};
             if (r == nt - 1) {
                 sh.taken_docs = excl + cnt;
                 if (cnt < sz) {
@@ -370,7 +370,8 @@ __global__ void __launch_bounds__(1024, 1) seismic_cluster_kernel(SeismicLaunch 
     __shared__ Shared sh;
     __shared__ int64_t slot_lb0[32];
     __shared__ int32_t slot_nb[32];
-    constexpr bool kRank = std::is_same<V, float>::value;
+    constexpr bool kRank = kRankTable<V, TE>;
+    constexpr bool kF32 = std::is_same<V, float>::value;
     constexpr int vsz = static_cast<int>(sizeof(V));
     cg::cluster_group cl = cg::this_cluster();
     const int rank = static_cast<int>(cl.block_rank()), ncl = static_cast<int>(cl.num_blocks());
@@ -454,9 +455,11 @@ __global__ void __launch_bounds__(1024, 1) seismic_cluster_kernel(SeismicLaunch 
                 if constexpr (kRank) tbl[t] = static_cast<TE>(i + 1);
                 else tbl[t] = static_cast<TE>(v);
             }
-            if constexpr (kRank) {
-                qv[i + 1] = ValT<V>::f(v);
-                bad |= !isfinite(ValT<V>::f(v));
+            if constexpr (kF32) {
+                qv[i + 1] = v;
+                bad |= !isfinite(v);
+            } else if constexpr (kRank) {
+                reinterpret_cast<uint32_t*>(qv)[i + 1] = v;
             }
         }
         const bool nonfinite = __syncthreads_or(bad) != 0;
@@ -581,7 +584,7 @@ __global__ void __launch_bounds__(1024, 1) seismic_cluster_kernel(SeismicLaunch 
                             // (the others copy the segments)
                             const int per = (total + ncl - 1) / ncl;
                             const int i1 = min(total, per);
-                            if (kRank && nonfinite)
+                            if (kF32 && nonfinite)
                                 score_share<V, TE, true>(a, sel, ctl, tbl, qv, cdoc, coff, clen, csc,
                                                          cseg, segs, nseg, 0, i1, tid, lane);
                             else
@@ -604,7 +607,7 @@ __global__ void __launch_bounds__(1024, 1) seismic_cluster_kernel(SeismicLaunch 
                         __syncthreads();
                         // the work counters: docs of segments the walk took
                         for (int i = tid; i < total; i += NT) {
-                            if (cdoc[i] >= 0 && !segs[cseg[i]].dropped) {
+                            if (cdoc[i] >= 0 && segs[cseg[i]].docs >= 0) {
                                 ++docs_scored;
                                 row_bytes += 8 + static_cast<int32_t>(clen[i]) * (2 + vsz);
                             }
@@ -635,7 +638,7 @@ __global__ void __launch_bounds__(1024, 1) seismic_cluster_kernel(SeismicLaunch 
                     __syncthreads();
                     const int per = (total + ncl - 1) / ncl;
                     const int i0 = min(total, rank * per), i1 = min(total, i0 + per);
-                    if (kRank && nonfinite)
+                    if (kF32 && nonfinite)
                         score_share<V, TE, true>(a, sel, ctl, tbl, qv, cdoc, coff, clen, csc, cseg,
                                                  segs, nseg, i0, i1, tid, lane);
                     else
@@ -738,7 +741,8 @@ cudaError_t launch_seismic_cluster(int val_kind, const SeismicLaunch& a, int war
         return a.qcap > 255 ? launch_typed<float, uint16_t>(a, warps, blocks, smem, placed, s)
                             : launch_typed<float, uint8_t>(a, warps, blocks, smem, placed, s);
     if (val_kind == kU8) return launch_typed<uint8_t, uint8_t>(a, warps, blocks, smem, placed, s);
-    return launch_typed<uint16_t, uint16_t>(a, warps, blocks, smem, placed, s);
+    return a.qcap > 255 ? launch_typed<uint16_t, uint16_t>(a, warps, blocks, smem, placed, s)
+                        : launch_typed<uint16_t, uint8_t>(a, warps, blocks, smem, placed, s);
 }
 
 }  // namespace nsp

@@ -8,7 +8,8 @@
 //      the reference's dimension-sized dense buffer (seismic_index.cpp:243-
 //      246), one byte per term: fp32 queries store the term's rank (0 = not
 //      in the query; the rank indexes a table of the query's values, entry 0
-//      holding 0.0f), SQ queries store the code itself;
+//      holding 0), 8-bit queries store the code itself, 16-bit queries the
+//      rank while a byte holds it;
 //   2. the query cut (utils/vector_process.h:18-30) is a rank selection;
 //   3. block summary scores (inverted_list_clusters.cpp:295-331) of up to
 //      one list per warp are accumulated at once, each warp hit term by hit
@@ -58,7 +59,8 @@ namespace {
 template <typename V, typename TE, int kG>
 __global__ void __launch_bounds__(1024, 1) seismic_cta_kernel(SeismicLaunch a) {
     extern __shared__ __align__(16) unsigned char smem[];
-    constexpr bool kRank = std::is_same<V, float>::value;
+    constexpr bool kRank = kRankTable<V, TE>;
+    constexpr bool kF32 = std::is_same<V, float>::value;
     constexpr int vsz = static_cast<int>(sizeof(V));
     const int tid = threadIdx.x;
     const int lane = tid & 31;
@@ -136,9 +138,11 @@ __global__ void __launch_bounds__(1024, 1) seismic_cta_kernel(SeismicLaunch a) {
                     tbl[t] = static_cast<TE>(v);
                 }
             }
-            if constexpr (kRank) {
-                qv[i + 1] = ValT<V>::f(v);
-                bad |= !isfinite(ValT<V>::f(v));
+            if constexpr (kF32) {
+                qv[i + 1] = v;
+                bad |= !isfinite(v);
+            } else if constexpr (kRank) {
+                reinterpret_cast<uint32_t*>(qv)[i + 1] = v;
             }
         }
         const bool nonfinite = __syncthreads_or(bad) != 0;
@@ -241,37 +245,78 @@ __global__ void __launch_bounds__(1024, 1) seismic_cta_kernel(SeismicLaunch a) {
                     }
                     __syncthreads();
                     const int nseg = ctl->nseg;
-                    const int total = ctl->total;
+                    int total = ctl->total;
                     if (nseg == 0) break;
                     if (total > 0) {
                         // candidates: doc ids and row info of every segment's docs
-                        for (int i = tid; i < total; i += blockDim.x) {
-                            int lo = 0, hi = nseg - 1;
-                            while (lo < hi) {
-                                const int mid = (lo + hi + 1) >> 1;
-                                if (segs[mid].cand0 <= i)
-                                    lo = mid;
-                                else
-                                    hi = mid - 1;
+                        // (with a selector: of its members, in order)
+                        int members = 0;
+                        for (int i0 = 0; i0 < total; i0 += blockDim.x) {
+                            const int i = i0 + tid;
+                            bool member = i < total;
+                            int32_t d = 0;
+                            int lo = 0, at = i;
+                            uint2 ri = make_uint2(0u, 0u);
+                            if (member) {
+                                int hi = nseg - 1;
+                                while (lo < hi) {
+                                    const int mid = (lo + hi + 1) >> 1;
+                                    if (segs[mid].cand0 <= i)
+                                        lo = mid;
+                                    else
+                                        hi = mid - 1;
+                                }
+                                const Seg& g = segs[lo];
+                                const int64_t pj = g.d0 + (i - g.cand0);
+                                d = __ldg(a.ix.docs + pj);
+                                // row info stored with the posting, else looked up
+                                ri = a.ix.drow != nullptr ? __ldg(a.ix.drow + pj)
+                                                          : __ldg(a.fwd.rowinfo + d);
+                                if (sel != nullptr)
+                                    member = (__ldg(sel + (d >> 6)) >> (d & 63)) & 1ull;
                             }
-                            const Seg& g = segs[lo];
-                            const int64_t pj = g.d0 + (i - g.cand0);
-                            const int32_t d = __ldg(a.ix.docs + pj);
-                            // row info stored with the posting, else looked up
-                            uint2 ri = a.ix.drow != nullptr ? __ldg(a.ix.drow + pj)
-                                                            : __ldg(a.fwd.rowinfo + d);
-                            bool member = true;
-                            if (sel != nullptr)
-                                member = (__ldg(sel + (d >> 6)) >> (d & 63)) & 1ull;
-                            if (!member) ri = make_uint2(0u, 0u);
-                            cdoc[i] = member ? d : -1;
-                            coff[i] = ri.x;
-                            clen[i] = ri.y;
-                            cseg[i] = static_cast<uint16_t>(lo);
+                            if (sel != nullptr) {
+                                const unsigned m = __ballot_sync(kFull, member);
+                                if (lane == 0) wsum[warp] = __popc(m);
+                                __syncthreads();
+                                at = members + __popc(m & ((1u << lane) - 1u));
+                                for (int w = 0; w < nwarps; ++w) {
+                                    const int c = wsum[w];
+                                    at += w < warp ? c : 0;
+                                    members += c;
+                                }
+                                __syncthreads();
+                            }
+                            if (member) {
+                                cdoc[at] = d;
+                                coff[at] = ri.x;
+                                clen[at] = ri.y;
+                                cseg[at] = static_cast<uint16_t>(lo);
+                            }
                         }
                         __syncthreads();
+                        if (sel != nullptr) {
+                            total = members;
+                            // the segments' members among the candidates
+                            for (int t = tid; t < nseg; t += blockDim.x) {
+                                int bound[2];
+#pragma unroll
+                                for (int u = 0; u < 2; ++u) {
+                                    int lo = 0, hi = total;
+                                    while (lo < hi) {
+                                        const int mid = (lo + hi) >> 1;
+                                        if (cseg[mid] < t + u) lo = mid + 1;
+                                        else hi = mid;
+                                    }
+                                    bound[u] = lo;
+                                }
+                                segs[t].cand0 = bound[0];
+                                segs[t].cnt = bound[1] - bound[0];
+                            }
+                            __syncthreads();
+                        }
                         // 6. scores
-                        if (kRank && nonfinite)
+                        if (kF32 && nonfinite)
                             score_batch<V, TE, true, kG>(a.fwd, ctl, tbl, qv, coff, clen, csc,
                                                          total, lane);
                         else
@@ -288,12 +333,10 @@ __global__ void __launch_bounds__(1024, 1) seismic_cta_kernel(SeismicLaunch a) {
                         const int nh = ctl->nheap;
                         const float hmin0 = nh == a.k ? hs[0] : 0.0f;
                         for (int i = tid; i < total; i += blockDim.x) {
-                            if (cdoc[i] >= 0) {
-                                ++docs_scored;
-                                row_bytes += 8 + static_cast<int32_t>(clen[i]) * (2 + vsz);
-                                if (nh < a.k || !(csc[i] <= hmin0))
-                                    atomicMax(&segs[cseg[i]].best, score_key(csc[i]));
-                            }
+                            ++docs_scored;
+                            row_bytes += 8 + static_cast<int32_t>(clen[i]) * (2 + vsz);
+                            if (nh < a.k || !(csc[i] <= hmin0))
+                                atomicMax(&segs[cseg[i]].best, score_key(csc[i]));
                         }
                         __syncthreads();
                     }
@@ -413,8 +456,6 @@ cudaError_t launch_cta_typed(const SeismicLaunch& a, int warps, int blocks, cuda
 
 }  // namespace
 
-// Table entries: fp32 queries hold ranks, one byte while the query has at
-// most 255 terms; SQ queries hold their codes.
 // Claim order of a batched launch: queries by row length, longest first (a
 // counting sort over lengths clamped to 255, one CTA).
 __global__ void __launch_bounds__(1024) order_by_length_kernel(const int32_t* indptr, int32_t n,
@@ -440,8 +481,11 @@ __global__ void __launch_bounds__(1024) order_by_length_kernel(const int32_t* in
     for (int32_t i = threadIdx.x; i < n; i += blockDim.x) order[atomicAdd(&bin[key(i)], 1)] = i;
 }
 
+// Table entries: fp32 and 16-bit queries hold ranks, one byte while the query
+// has at most 255 terms; else two bytes (fp32: ranks, 16-bit: codes). 8-bit
+// queries hold their codes.
 static bool wide_table(int val_kind, int qcap) {
-    return val_kind == kU16 || (val_kind == kF32 && qcap > 255);
+    return (val_kind == kU16 || val_kind == kF32) && qcap > 255;
 }
 
 size_t seismic_cta_smem(int val_kind, int dim, int qcap, int k, int batch, int seg_cap) {
@@ -450,7 +494,9 @@ size_t seismic_cta_smem(int val_kind, int dim, int qcap, int k, int batch, int s
                    ? smem_typed<float, uint16_t>(dim, qcap, k, batch, seg_cap)
                    : smem_typed<float, uint8_t>(dim, qcap, k, batch, seg_cap);
     if (val_kind == kU8) return smem_typed<uint8_t, uint8_t>(dim, qcap, k, batch, seg_cap);
-    return smem_typed<uint16_t, uint16_t>(dim, qcap, k, batch, seg_cap);
+    return wide_table(val_kind, qcap)
+               ? smem_typed<uint16_t, uint16_t>(dim, qcap, k, batch, seg_cap)
+               : smem_typed<uint16_t, uint8_t>(dim, qcap, k, batch, seg_cap);
 }
 
 int seismic_cta_seg_cap(int cluster) { return cluster > 1 ? kSegCapMax : kSegCap; }
@@ -462,7 +508,8 @@ int seismic_cta_max_blocks_per_sm(int val_kind, int qcap, int group, int warps, 
                    ? max_blocks_cta_typed<float, uint16_t>(group, th, smem)
                    : max_blocks_cta_typed<float, uint8_t>(group, th, smem);
     if (val_kind == kU8) return max_blocks_cta_typed<uint8_t, uint8_t>(group, th, smem);
-    return max_blocks_cta_typed<uint16_t, uint16_t>(group, th, smem);
+    return wide_table(val_kind, qcap) ? max_blocks_cta_typed<uint16_t, uint16_t>(group, th, smem)
+                                      : max_blocks_cta_typed<uint16_t, uint8_t>(group, th, smem);
 }
 
 cudaError_t launch_seismic_cta(int val_kind, const SeismicLaunch& launch, int warps, int blocks,
@@ -482,7 +529,8 @@ cudaError_t launch_seismic_cta(int val_kind, const SeismicLaunch& launch, int wa
         return wide_table(val_kind, a.qcap) ? launch_cta_typed<float, uint16_t>(a, warps, blocks, s)
                                             : launch_cta_typed<float, uint8_t>(a, warps, blocks, s);
     if (val_kind == kU8) return launch_cta_typed<uint8_t, uint8_t>(a, warps, blocks, s);
-    return launch_cta_typed<uint16_t, uint16_t>(a, warps, blocks, s);
+    return wide_table(val_kind, a.qcap) ? launch_cta_typed<uint16_t, uint16_t>(a, warps, blocks, s)
+                                        : launch_cta_typed<uint16_t, uint8_t>(a, warps, blocks, s);
 }
 
 cudaError_t launch_order_by_length(const int32_t* indptr, int32_t n, int32_t* order,

@@ -31,12 +31,12 @@ constexpr int kSegCapMax = 1024;  // the most any launch asks for (a cluster per
 // A run of consecutive docs of one block inside a batch.
 struct Seg {
     int64_t d0;     // position of the first doc in ix.docs
-    int32_t cnt;    // docs in the segment
+    int32_t cnt;    // its candidates (with a selector, its member docs)
     int32_t cand0;  // first candidate slot of the batch
     float bs;       // the block's summary score
     int32_t head;   // 1 when the block starts here (its pruning test applies)
     uint32_t best;  // key of its best member score above the heap minimum at the gather (0: none)
-    int32_t dropped;  // 1 when the walk dropped it (the cluster kernel's counters)
+    int32_t docs;   // docs in the segment; the cluster kernel's walk sets -1 when it drops it
 };
 
 // Order-preserving keys of scores, above 0 (NaN sorts past every number: a
@@ -225,10 +225,20 @@ __device__ __forceinline__ int partial_steps(const uint16_t* ip, const uint8_t* 
     return (acc[0] + acc[1]) + (acc[2] + acc[3]);
 }
 
-// uint16 codes: int64 sum (distance.h:49-57).
+// What a query's table holds per term: the term's rank among the query's
+// terms (an index into the query's values), or its code. fp32 values need the
+// rank; 16-bit codes take it while a byte holds it, since a table of codes is
+// 61 KB for 30,522 terms and leaves room for two CTAs per SM instead of four
+// (1,001 queries on 301,000 docs: 8.8 ms with codes, 6.6 ms with ranks).
+template <typename V, typename TE>
+constexpr bool kRankTable = std::is_same<V, float>::value ||
+                            (std::is_same<V, uint16_t>::value && std::is_same<TE, uint8_t>::value);
+
+// uint16 codes: int64 sum (distance.h:49-57). `qv`: the query's codes by
+// rank (32-bit words), for a table of ranks.
 template <typename TE>
 __device__ __forceinline__ long long partial(const uint16_t* ip, const uint16_t* vp, int rem,
-                                             const TE* tbl) {
+                                             const TE* tbl, const float* qv) {
     if (rem <= 0) return 0;
     uint32_t t[8], v[8];
     ldg256(ip, t);
@@ -236,9 +246,12 @@ __device__ __forceinline__ long long partial(const uint16_t* ip, const uint16_t*
     long long acc = 0;
 #pragma unroll
     for (int u = 0; u < 16; ++u) {
-        const unsigned long long q = static_cast<unsigned long long>(tbl[term_of(t, u)]);
-        const unsigned long long x = static_cast<unsigned long long>(term_of(v, u));
-        acc += static_cast<long long>(x * q);
+        uint32_t q;
+        if constexpr (kRankTable<uint16_t, TE>)
+            q = reinterpret_cast<const uint32_t*>(qv)[tbl[term_of(t, u)]];
+        else
+            q = tbl[term_of(t, u)];
+        acc += static_cast<long long>(static_cast<unsigned long long>(term_of(v, u)) * q);
     }
     return acc;
 }
@@ -350,7 +363,7 @@ __device__ void score_batch(const FwdView& fwd, Ctl* ctl, const TE* tbl, const f
         } else if constexpr (kU8) {
             acc += group_sum<kG>(partial_steps<TE, kU8Steps>(ip, vp, mine, 16 * kG, tbl));
         } else {
-            acc += group_sum<kG>(partial<TE>(ip, vp, mine, tbl));
+            acc += group_sum<kG>(partial<TE>(ip, vp, mine, tbl, qv));
         }
         if (act) {
             ip += kStep;
@@ -697,6 +710,7 @@ __device__ int gather(const SeismicLaunch& a, Cursor& c, bool first, int64_t lb0
             Seg g;
             g.d0 = c.split_d;
             g.cnt = take;
+            g.docs = take;
             g.cand0 = 0;
             g.bs = c.split_bs;
             g.head = 0;
@@ -754,6 +768,7 @@ __device__ int gather(const SeismicLaunch& a, Cursor& c, bool first, int64_t lb0
             Seg g;
             g.d0 = d0;
             g.cnt = min(sz, room - excl);
+            g.docs = g.cnt;
             g.cand0 = total + excl;
             g.bs = bs;
             g.head = 1;
@@ -841,7 +856,7 @@ __device__ __forceinline__ void walk_batch(const SeismicLaunch& a, Seg* segs, in
     // a lone query drops hundreds at once).
     auto drop = [&](int s0, int s1) {
         if constexpr (kMark) {
-            for (int t = s0 + lane; t < s1; t += 32) segs[t].dropped = 1;
+            for (int t = s0 + lane; t < s1; t += 32) segs[t].docs = -1;
         } else {
             const int c1 = s1 < nseg ? segs[s1].cand0 : total;
             for (int i = segs[s0].cand0 + lane; i < c1; i += 32) {
@@ -912,7 +927,7 @@ __device__ __forceinline__ void walk_batch(const SeismicLaunch& a, Seg* segs, in
     bool ended = false;
     for (int s0 = 0; s0 < nseg && !ended; s0 += 32) {
         const bool valid = s0 + lane < nseg;
-        int head = 0, cnt = 0, cand0 = 0;
+        int head = 0, cnt = 0, cand0 = 0, docs = 0;
         uint32_t best = 0u;
         float bs = 0.0f;
         if (valid) {
@@ -920,6 +935,7 @@ __device__ __forceinline__ void walk_batch(const SeismicLaunch& a, Seg* segs, in
             head = g.head;
             cnt = g.cnt;
             cand0 = g.cand0;
+            docs = g.docs;
             best = g.best;
             bs = g.bs;
         }
@@ -943,7 +959,7 @@ __device__ __forceinline__ void walk_batch(const SeismicLaunch& a, Seg* segs, in
             const int heads = __popc(__ballot_sync(kFull, taken && head));
             blocks_visited += heads;
             bytes += 16u * heads +
-                     4u * __reduce_add_sync(kFull, taken ? cnt : 0);
+                     4u * __reduce_add_sync(kFull, taken ? docs : 0);
             if (a.visit != nullptr) {
                 unsigned tm = __ballot_sync(kFull, taken);
                 while (tm) {
@@ -985,7 +1001,7 @@ __device__ __forceinline__ void walk_batch(const SeismicLaunch& a, Seg* segs, in
                     ++blocks_visited;
                     bytes += 16;
                 }
-                bytes += 4u * static_cast<uint32_t>(gcnt);
+                bytes += 4u * static_cast<uint32_t>(__shfl_sync(kFull, docs, pos));
                 count_visits(s0 + pos);
                 for (int b = 0; b < gcnt; b += 128) {
                     // four times 32 docs loaded at once
