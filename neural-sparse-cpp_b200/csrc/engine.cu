@@ -25,22 +25,36 @@ void cuda_check(cudaError_t e, const char* what) {
     }
 }
 
-int device_sm_count() {
+namespace {
+// A device attribute, looked up once per device.
+int device_attribute(cudaDeviceAttr a, std::atomic<int>* known) {
+    constexpr int kDevices = 64;
     int dev = 0;
     cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
-    int sms = 0;
-    cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev),
-               "cudaDeviceGetAttribute");
-    return sms;
+    if (dev < kDevices) {
+        const int v = known[dev].load(std::memory_order_relaxed);
+        if (v > 0) return v;
+    }
+    int v = 0;
+    cuda_check(cudaDeviceGetAttribute(&v, a, dev), "cudaDeviceGetAttribute");
+    if (dev < kDevices) known[dev].store(v, std::memory_order_relaxed);
+    return v;
+}
+}  // namespace
+
+int device_sm_count() {
+    static std::atomic<int> known[64];
+    return device_attribute(cudaDevAttrMultiProcessorCount, known);
 }
 
 static int max_smem_optin() {
-    int dev = 0;
-    cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
-    int v = 0;
-    cuda_check(cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev),
-               "cudaDeviceGetAttribute");
-    return v;
+    static std::atomic<int> known[64];
+    return device_attribute(cudaDevAttrMaxSharedMemoryPerBlockOptin, known);
+}
+
+static int max_smem_per_sm() {
+    static std::atomic<int> known[64];
+    return device_attribute(cudaDevAttrMaxSharedMemoryPerMultiprocessor, known);
 }
 
 // ---------------------------------------------------------------- arena --
@@ -74,15 +88,6 @@ void* Arena::bytes(size_t n) {
     return p;
 }
 
-static int max_smem_per_sm() {
-    int dev = 0;
-    cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
-    int v = 0;
-    cuda_check(cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev),
-               "cudaDeviceGetAttribute");
-    return v;
-}
-
 // ------------------------------------------------------------ workspace --
 
 Workspace::Workspace() {
@@ -97,7 +102,14 @@ Workspace::~Workspace() {
         if (dptr_[i] != nullptr) cudaFree(dptr_[i]);
         if (hptr_[i] != nullptr) cudaFreeHost(hptr_[i]);
     }
+    for (cudaEvent_t e : event_)
+        if (e != nullptr) cudaEventDestroy(e);
     if (stream_ != nullptr) cudaStreamDestroy(stream_);
+}
+
+cudaEvent_t Workspace::event(int i) {
+    if (event_[i] == nullptr) cuda_check(cudaEventCreate(&event_[i]), "event");
+    return event_[i];
 }
 
 Workspace& Workspace::get() {
@@ -502,27 +514,38 @@ struct Uploaded {
     int64_t nnz;
 };
 
+// A batch's staging block: offsets of the terms and values after the row
+// pointers (16-byte aligned, with 16 bytes past each array).
+struct QueryBytes {
+    size_t idx, val, total;
+};
+QueryBytes query_bytes(int64_t n, int64_t nnz) {
+    auto up = [](size_t x) { return (x + 31) & ~size_t(15); };
+    QueryBytes b;
+    b.idx = up((static_cast<size_t>(n) + 1) * sizeof(int32_t));
+    b.val = b.idx + up(static_cast<size_t>(nnz) * sizeof(uint16_t));
+    b.total = b.val + up(static_cast<size_t>(nnz) * sizeof(float));
+    return b;
+}
+
 Uploaded upload_queries(Workspace& ws, const QueryBatch& q) {
     cudaStream_t s = ws.stream();
     const int64_t nnz = q.ip[q.n] - q.ip[0];
     Uploaded u;
     u.nnz = nnz;
-    auto* hi = static_cast<int32_t*>(ws.pinned(Workspace::kQIndptr, (q.n + 1) * sizeof(int32_t)));
-    auto* hx = static_cast<uint16_t*>(ws.pinned(Workspace::kQIdx, nnz * sizeof(uint16_t)));
-    auto* hv = static_cast<float*>(ws.pinned(Workspace::kQVal, nnz * sizeof(float)));
+    // one staging block and one copy: row pointers, terms, values
+    const QueryBytes b = query_bytes(q.n, nnz);
+    auto* h = static_cast<unsigned char*>(ws.pinned(Workspace::kQuery, b.total));
+    auto* d = static_cast<unsigned char*>(ws.dev(Workspace::kQuery, b.total));
+    auto* hi = reinterpret_cast<int32_t*>(h);
     const int32_t base = q.ip[0];
     for (int32_t i = 0; i <= q.n; ++i) hi[i] = q.ip[i] - base;
-    std::memcpy(hx, q.ix + base, nnz * sizeof(uint16_t));
-    std::memcpy(hv, q.vv + base, nnz * sizeof(float));
-    u.indptr = static_cast<int32_t*>(ws.dev(Workspace::kQIndptr, (q.n + 1) * sizeof(int32_t)));
-    u.idx = static_cast<uint16_t*>(ws.dev(Workspace::kQIdx, nnz * sizeof(uint16_t) + 16));
-    u.val = static_cast<float*>(ws.dev(Workspace::kQVal, nnz * sizeof(float) + 16));
-    cuda_check(cudaMemcpyAsync(u.indptr, hi, (q.n + 1) * sizeof(int32_t), cudaMemcpyHostToDevice, s),
-               "H2D queries");
-    cuda_check(cudaMemcpyAsync(u.idx, hx, nnz * sizeof(uint16_t), cudaMemcpyHostToDevice, s),
-               "H2D queries");
-    cuda_check(cudaMemcpyAsync(u.val, hv, nnz * sizeof(float), cudaMemcpyHostToDevice, s),
-               "H2D queries");
+    std::memcpy(h + b.idx, q.ix + base, nnz * sizeof(uint16_t));
+    std::memcpy(h + b.val, q.vv + base, nnz * sizeof(float));
+    u.indptr = reinterpret_cast<int32_t*>(d);
+    u.idx = reinterpret_cast<uint16_t*>(d + b.idx);
+    u.val = reinterpret_cast<float*>(d + b.val);
+    cuda_check(cudaMemcpyAsync(d, h, b.total, cudaMemcpyHostToDevice, s), "H2D queries");
     return u;
 }
 
@@ -536,17 +559,34 @@ const uint64_t* upload_sel(Workspace& ws, const std::vector<uint64_t>* sel) {
     return d;
 }
 
-void download_results(Workspace& ws, int32_t n, int k, const float* dd, const int32_t* dl,
-                      float* out_d, int32_t* out_l) {
-    cudaStream_t s = ws.stream();
+// Results on the device, scores then labels, so one copy brings both.
+struct Results {
+    float* d;
+    int32_t* l;
+    size_t count;
+};
+Results result_block(Workspace& ws, int32_t n, int k) {
     const size_t cnt = static_cast<size_t>(n) * k;
-    auto* hd = static_cast<float*>(ws.pinned(Workspace::kOutD, cnt * sizeof(float)));
-    auto* hl = static_cast<int32_t*>(ws.pinned(Workspace::kOutL, cnt * sizeof(int32_t)));
-    cuda_check(cudaMemcpyAsync(hd, dd, cnt * sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
-    cuda_check(cudaMemcpyAsync(hl, dl, cnt * sizeof(int32_t), cudaMemcpyDeviceToHost, s), "D2H");
+    auto* d = static_cast<float*>(ws.dev(Workspace::kOut, cnt * 8));
+    return {d, reinterpret_cast<int32_t*>(d + cnt), cnt};
+}
+
+// Copies the results, and `extra` bytes at `src` into pinned memory where not
+// null, waits once and hands the results out.
+void download_results(Workspace& ws, const Results& r, float* out_d, int32_t* out_l,
+                      const void* src = nullptr, size_t extra = 0, const void* src2 = nullptr,
+                      size_t extra2 = 0) {
+    cudaStream_t s = ws.stream();
+    auto* h = static_cast<unsigned char*>(ws.pinned(Workspace::kOut, r.count * 8));
+    auto* c = static_cast<unsigned char*>(ws.pinned(Workspace::kStats, 256));
+    cuda_check(cudaMemcpyAsync(h, r.d, r.count * 8, cudaMemcpyDeviceToHost, s), "D2H");
+    if (src != nullptr)
+        cuda_check(cudaMemcpyAsync(c, src, extra, cudaMemcpyDeviceToHost, s), "D2H");
+    if (src2 != nullptr)
+        cuda_check(cudaMemcpyAsync(c + 128, src2, extra2, cudaMemcpyDeviceToHost, s), "D2H");
     cuda_check(cudaStreamSynchronize(s), "search sync");
-    std::memcpy(out_d, hd, cnt * sizeof(float));
-    std::memcpy(out_l, hl, cnt * sizeof(int32_t));
+    std::memcpy(out_d, h, r.count * sizeof(float));
+    std::memcpy(out_l, h + r.count * sizeof(float), r.count * sizeof(int32_t));
 }
 
 int val_kind_of(int qbits) { return qbits == 0 ? kF32 : (qbits == 8 ? kU8 : kU16); }
@@ -678,10 +718,10 @@ constexpr int kDefaultVariant = 4;
 
 }  // namespace
 
-void run_seismic(const ForwardDevice& fwd, const SeismicDevice& ix, int32_t n,
-                 const int32_t* d_indptr, const uint16_t* d_idx, const void* d_vals, int32_t qcap,
-                 const SeismicSearchArgs& args_in, const uint64_t* d_sel, float* d_out,
-                 int32_t* d_lab, cudaStream_t s, Scratch& ws, SearchStats* stats) {
+int run_seismic(const ForwardDevice& fwd, const SeismicDevice& ix, int32_t n,
+                const int32_t* d_indptr, const uint16_t* d_idx, const void* d_vals, int32_t qcap,
+                const SeismicSearchArgs& args_in, const uint64_t* d_sel, float* d_out,
+                int32_t* d_lab, cudaStream_t s, Scratch& ws, bool timed) {
     SeismicSearchArgs args = args_in;
     if (args.variant < 0) args.variant = kDefaultVariant;
     if (args.d_sel_q != nullptr && args.variant < 2)
@@ -708,18 +748,14 @@ void run_seismic(const ForwardDevice& fwd, const SeismicDevice& ix, int32_t n,
     a.out_l = d_lab;
     a.qcap = std::max(qcap, 1);
     a.nnz_cap = args.nnz_cap;
-    auto* st = static_cast<unsigned long long*>(
-        ws.dev(Workspace::kStats, kStatCount * sizeof(unsigned long long)));
-    cuda_check(cudaMemsetAsync(st, 0, kStatCount * sizeof(unsigned long long), s), "memset");
+    // the work counters and, after them, the claim counter
+    auto* st = static_cast<unsigned long long*>(ws.dev(Workspace::kStats, kControlBytes));
+    cuda_check(cudaMemsetAsync(st, 0, kControlBytes, s), "memset");
     a.stats = st;
     // The kernel's own time, only when asked for: an event recorded inside a
     // stream capture would outlive this call in the graph.
-    const bool timed = stats != nullptr;
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
-    if (timed) {
-        cuda_check(cudaEventCreate(&e0), "event");
-        cuda_check(cudaEventCreate(&e1), "event");
-    }
+    const cudaEvent_t e0 = timed ? Workspace::get().event(0) : nullptr;
+    const cudaEvent_t e1 = timed ? Workspace::get().event(1) : nullptr;
     auto mark = [&](cudaEvent_t e) {
         if (timed) cuda_check(cudaEventRecord(e, s), "event");
     };
@@ -770,8 +806,7 @@ void run_seismic(const ForwardDevice& fwd, const SeismicDevice& ix, int32_t n,
                        static_cast<size_t>(p.blocks) * p2 * sizeof(unsigned long long)));
         }
         if (!args.plain) {
-            a.work_counter = static_cast<int32_t*>(ws.dev(Workspace::kCounter, sizeof(int32_t)));
-            cuda_check(cudaMemsetAsync(a.work_counter, 0, sizeof(int32_t), s), "memset");
+            a.work_counter = reinterpret_cast<int32_t*>(st + kStatCount);
             a.first_query = 0;
             // more queries than CTAs: the longest rows are claimed first, so
             // the launch does not end on a long query claimed last (16,384
@@ -809,8 +844,7 @@ void run_seismic(const ForwardDevice& fwd, const SeismicDevice& ix, int32_t n,
         const size_t warps = static_cast<size_t>(p.blocks) * p.wpb;
         a.bscore = static_cast<float*>(
             ws.dev(Workspace::kBScore, warps * one_warp_slot(a.ix.max_blocks) * sizeof(float)));
-        a.work_counter = static_cast<int32_t*>(ws.dev(Workspace::kCounter, sizeof(int32_t)));
-        cuda_check(cudaMemsetAsync(a.work_counter, 0, sizeof(int32_t), s), "memset");
+        a.work_counter = reinterpret_cast<int32_t*>(st + kStatCount);
         a.first_query = 0;
         mark(e0);
         cuda_check(launch_seismic(kind, a, p.wpb, p.blocks, s), "seismic search launch");
@@ -837,27 +871,29 @@ void run_seismic(const ForwardDevice& fwd, const SeismicDevice& ix, int32_t n,
         mark(e1);
         launches = n;
     }
-    if (stats != nullptr) {
-        unsigned long long h[kStatCount];
-        cuda_check(cudaMemcpyAsync(h, st, sizeof(h), cudaMemcpyDeviceToHost, s), "D2H stats");
-        cuda_check(cudaStreamSynchronize(s), "sync");
-        float ms = 0.0f;
-        cuda_check(cudaEventElapsedTime(&ms, e0, e1), "event time");
-        stats->docs_scored = h[kStatDocsScored];
-        stats->blocks_visited = h[kStatBlocksVisited];
-        stats->bytes = h[kStatBytes];
-        stats->lists_probed = h[kStatListsProbed];
-        stats->kernel_ms = ms;
-        stats->launches = launches;
-        stats->row_bytes = h[kStatRowBytes];
-        stats->unique_docs = h[kStatUniqueDocs];
-        stats->unique_row_bytes = h[kStatUniqueRowBytes];
-    }
-    if (timed) {
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-    }
+    return launches;
 }
+
+namespace {
+
+// The counters of a finished search, from its control block in pinned memory
+// (download_results) and the thread's events.
+void read_stats(Workspace& ws, int launches, SearchStats* stats) {
+    const auto* h = static_cast<const unsigned long long*>(ws.pinned(Workspace::kStats, 256));
+    float ms = 0.0f;
+    cuda_check(cudaEventElapsedTime(&ms, ws.event(0), ws.event(1)), "event time");
+    stats->docs_scored = h[kStatDocsScored];
+    stats->blocks_visited = h[kStatBlocksVisited];
+    stats->bytes = h[kStatBytes];
+    stats->lists_probed = h[kStatListsProbed];
+    stats->kernel_ms = ms;
+    stats->launches = launches;
+    stats->row_bytes = h[kStatRowBytes];
+    stats->unique_docs = h[kStatUniqueDocs];
+    stats->unique_row_bytes = h[kStatUniqueRowBytes];
+}
+
+}  // namespace
 
 SeismicScratchNeed seismic_scratch_need(const ForwardDevice& fwd, const SeismicDevice& ix,
                                         int32_t n, int32_t max_nnz,
@@ -869,9 +905,9 @@ SeismicScratchNeed seismic_scratch_need(const ForwardDevice& fwd, const SeismicD
     const int qcap = std::max(max_nnz, 1);
     const int maxb = std::max(ix.max_blocks(), 1);
     SeismicScratchNeed need;
-    // stats, error word, work counter (run_seismic asks for each), and the
+    // control block and error word (run_seismic asks for each), and the
     // claim order of a batched launch of the one-CTA-per-query kernels
-    need.fixed = kStatCount * sizeof(unsigned long long) + 2 * sizeof(int32_t);
+    need.fixed = kControlBytes + sizeof(int32_t);
     if (args.variant >= 2) need.fixed += static_cast<size_t>(n) * sizeof(int32_t);
     if (args.variant >= 2) {
         const SeismicPlan p = plan_seismic_cta(kind, fwd.view().dim, qcap, args.k, n, args, false,
@@ -903,20 +939,15 @@ void reserve_seismic_scratch(const ForwardDevice& fwd, const SeismicDevice& ix, 
     const size_t nnz = nq * static_cast<size_t>(std::max(max_nnz, 1));
     const size_t cnt = nq * static_cast<size_t>(args.k);
     // the sizes upload_queries, download_results and run_seismic ask for
-    ws.pinned(Workspace::kQIndptr, (nq + 1) * sizeof(int32_t));
-    ws.pinned(Workspace::kQIdx, nnz * sizeof(uint16_t));
-    ws.pinned(Workspace::kQVal, nnz * sizeof(float));
-    ws.pinned(Workspace::kOutD, cnt * sizeof(float));
-    ws.pinned(Workspace::kOutL, cnt * sizeof(int32_t));
-    ws.dev(Workspace::kQIndptr, (nq + 1) * sizeof(int32_t));
-    ws.dev(Workspace::kQIdx, nnz * sizeof(uint16_t) + 16);
-    ws.dev(Workspace::kQVal, nnz * sizeof(float) + 16);
+    const size_t qb = query_bytes(n, static_cast<int64_t>(nnz)).total;
+    ws.pinned(Workspace::kQuery, qb);
+    ws.pinned(Workspace::kOut, cnt * 8);
+    ws.pinned(Workspace::kStats, 256);
+    ws.dev(Workspace::kQuery, qb);
     if (args.qbits != 0) ws.dev(Workspace::kQCode, nnz * 2 + 16);
-    ws.dev(Workspace::kOutD, cnt * sizeof(float));
-    ws.dev(Workspace::kOutL, cnt * sizeof(int32_t));
-    ws.dev(Workspace::kStats, kStatCount * sizeof(unsigned long long));
+    ws.dev(Workspace::kOut, cnt * 8);
+    ws.dev(Workspace::kStats, kControlBytes);
     ws.dev(Workspace::kErr, sizeof(int32_t));
-    ws.dev(Workspace::kCounter, sizeof(int32_t));
     if (args.variant < 2) return;
     const SeismicPlan p = plan_seismic_cta(val_kind_of(args.qbits), fwd.view().dim,
                                            std::max(max_nnz, 1), args.k, n, args, args.plain, false);
@@ -938,15 +969,19 @@ namespace {
 // Raises if a search kernel on `s` flagged an error (call after sync):
 // 1 a bounded wait gave up, 2 a sort buffer was missing, 3 a query longer
 // than the launch's query capacity.
+void raise_kernel_error(int32_t h) {
+    if (h == 1) throw std::runtime_error("search kernel gave up waiting for a bulk copy");
+    if (h == 2) throw std::runtime_error("search kernel had no buffer to sort a list's blocks");
+    if (h == 3) throw std::invalid_argument("a query row is longer than max_nnz");
+    if (h != 0) throw std::runtime_error("search kernel reported an error");
+}
+
 void check_kernel_error(Scratch& ws, cudaStream_t s) {
     int32_t h = 0;
     auto* err = static_cast<int32_t*>(ws.dev(Workspace::kErr, sizeof(int32_t)));
     cuda_check(cudaMemcpyAsync(&h, err, sizeof(int32_t), cudaMemcpyDeviceToHost, s), "D2H");
     cuda_check(cudaStreamSynchronize(s), "sync");
-    if (h == 1) throw std::runtime_error("search kernel gave up waiting for a bulk copy");
-    if (h == 2) throw std::runtime_error("search kernel had no buffer to sort a list's blocks");
-    if (h == 3) throw std::invalid_argument("a query row is longer than max_nnz");
-    if (h != 0) throw std::runtime_error("search kernel reported an error");
+    raise_kernel_error(h);
 }
 
 }  // namespace
@@ -965,12 +1000,17 @@ void seismic_search(const ForwardDevice& fwd, const SeismicDevice& ix, const Que
         vals = codes;
     }
     const uint64_t* d_sel = upload_sel(ws, sel_bits);
-    const size_t cnt = static_cast<size_t>(q.n) * args.k;
-    auto* dd = static_cast<float*>(ws.dev(Workspace::kOutD, cnt * sizeof(float)));
-    auto* dl = static_cast<int32_t*>(ws.dev(Workspace::kOutL, cnt * sizeof(int32_t)));
-    run_seismic(fwd, ix, q.n, u.indptr, u.idx, vals, q.max_nnz, args, d_sel, dd, dl, s, ws, stats);
-    download_results(ws, q.n, args.k, dd, dl, out_d, out_l);
-    check_kernel_error(ws, s);
+    const Results r = result_block(ws, q.n, args.k);
+    const int launches = run_seismic(fwd, ix, q.n, u.indptr, u.idx, vals, q.max_nnz, args, d_sel,
+                                     r.d, r.l, s, ws, stats != nullptr);
+    // results, counters and error word after one wait
+    download_results(ws, r, out_d, out_l, ws.dev(Workspace::kStats, kControlBytes), kControlBytes,
+                     ws.dev(Workspace::kErr, sizeof(int32_t)), sizeof(int32_t));
+    if (stats != nullptr) read_stats(ws, launches, stats);
+    int32_t err = 0;
+    std::memcpy(&err, static_cast<unsigned char*>(ws.pinned(Workspace::kStats, 256)) + 128,
+                sizeof(err));
+    raise_kernel_error(err);
 }
 
 void seismic_search_start(const ForwardDevice& fwd, const SeismicDevice& ix, const QueryBatch& q,
@@ -993,7 +1033,7 @@ void seismic_search_start(const ForwardDevice& fwd, const SeismicDevice& ix, con
         vals = codes;
     }
     run_seismic(fwd, ix, q.n, u.indptr, u.idx, vals, q.max_nnz, args, nullptr, out_d, out_l, s,
-                ws, nullptr);
+                ws, false);
 }
 
 void seismic_search_wait() {
@@ -1004,10 +1044,10 @@ void seismic_search_wait() {
 void seismic_search_device(const ForwardDevice& fwd, const SeismicDevice& ix, int32_t n,
                            const int32_t* d_indptr, const uint16_t* d_idx, const void* d_val,
                            int32_t max_nnz, const SeismicSearchArgs& args, const uint64_t* d_sel,
-                           float* d_out, int32_t* d_lab, cudaStream_t s, SearchStats* stats) {
+                           float* d_out, int32_t* d_lab, cudaStream_t s) {
     Workspace& ws = Workspace::get();
     run_seismic(fwd, ix, n, d_indptr, d_idx, d_val, max_nnz, args, d_sel, d_out, d_lab, s, ws,
-                stats);
+                false);
 }
 
 void exact_search(const ForwardDevice& fwd, const PostingsDevice* post, const QueryBatch& q, int k,
@@ -1017,9 +1057,10 @@ void exact_search(const ForwardDevice& fwd, const PostingsDevice* post, const Qu
     cudaStream_t s = ws.stream();
     const Uploaded u = upload_queries(ws, q);
     const uint64_t* d_sel = upload_sel(ws, sel_bits);
-    const size_t cnt = static_cast<size_t>(q.n) * k;
-    auto* dd = static_cast<float*>(ws.dev(Workspace::kOutD, cnt * sizeof(float)));
-    auto* dl = static_cast<int32_t*>(ws.dev(Workspace::kOutL, cnt * sizeof(int32_t)));
+    const Results r = result_block(ws, q.n, k);
+    const size_t cnt = r.count;
+    float* dd = r.d;
+    int32_t* dl = r.l;
 
     ExactLaunch a{};
     a.fwd = fwd.view();
@@ -1072,13 +1113,10 @@ void exact_search(const ForwardDevice& fwd, const PostingsDevice* post, const Qu
                                                              a.qcap * sizeof(float)))
                             : nullptr;
     }
-    auto* st = static_cast<unsigned long long*>(
-        ws.dev(Workspace::kStats, kStatCount * sizeof(unsigned long long)));
-    cuda_check(cudaMemsetAsync(st, 0, kStatCount * sizeof(unsigned long long), s), "memset");
+    auto* st = static_cast<unsigned long long*>(ws.dev(Workspace::kStats, kControlBytes));
+    cuda_check(cudaMemsetAsync(st, 0, kControlBytes, s), "memset");
     a.stats = st;
-    cudaEvent_t e0, e1;
-    cuda_check(cudaEventCreate(&e0), "event");
-    cuda_check(cudaEventCreate(&e1), "event");
+    const cudaEvent_t e0 = ws.event(0), e1 = ws.event(1);
     cuda_check(cudaEventRecord(e0, s), "event");
     if (fwd.n_docs() > 0) {
         cuda_check(taat ? launch_exact_taat(a, s) : launch_exact(a, tiles, s),
@@ -1087,6 +1125,7 @@ void exact_search(const ForwardDevice& fwd, const PostingsDevice* post, const Qu
         cuda_check(cudaMemsetAsync(dd, 0, cnt * sizeof(float), s), "memset");
     }
     cuda_check(cudaEventRecord(e1, s), "event");
+    SearchStats found;
     if (fwd.n_docs() == 0) {
         // nothing indexed: every slot is padding
         cuda_check(cudaStreamSynchronize(s), "sync");
@@ -1095,20 +1134,14 @@ void exact_search(const ForwardDevice& fwd, const PostingsDevice* post, const Qu
             out_l[i] = -1;
         }
     } else {
-        download_results(ws, q.n, k, dd, dl, out_d, out_l);
+        download_results(ws, r, out_d, out_l, st, kControlBytes);
+        read_stats(ws, 2, &found);
     }
     if (stats != nullptr) {
-        unsigned long long h[kStatCount];
-        cuda_check(cudaMemcpyAsync(h, st, sizeof(h), cudaMemcpyDeviceToHost, s), "D2H stats");
-        cuda_check(cudaStreamSynchronize(s), "sync");
-        float ms = 0.0f;
-        cuda_check(cudaEventElapsedTime(&ms, e0, e1), "event time");
-        stats->bytes = h[kStatBytes];
-        stats->kernel_ms = ms;
+        stats->bytes = found.bytes;
+        stats->kernel_ms = found.kernel_ms;
         stats->launches = 2;
     }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
 }
 
 void exact_list_search(const ForwardDevice& fwd, const QueryBatch& q, const SeismicSearchArgs& args,
@@ -1128,9 +1161,7 @@ void exact_list_search(const ForwardDevice& fwd, const QueryBatch& q, const Seis
     auto* did = static_cast<int32_t*>(ws.dev(Workspace::kIds, ids.size() * sizeof(int32_t) + 4));
     cuda_check(cudaMemcpyAsync(did, hid, ids.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s),
                "H2D ids");
-    const size_t cnt = static_cast<size_t>(q.n) * args.k;
-    auto* dd = static_cast<float*>(ws.dev(Workspace::kOutD, cnt * sizeof(float)));
-    auto* dl = static_cast<int32_t*>(ws.dev(Workspace::kOutL, cnt * sizeof(int32_t)));
+    const Results r = result_block(ws, q.n, args.k);
     QueryView qv;
     qv.n = q.n;
     qv.indptr = u.indptr;
@@ -1138,9 +1169,9 @@ void exact_list_search(const ForwardDevice& fwd, const QueryBatch& q, const Seis
     qv.val = vals;
     cuda_check(launch_exact_list(val_kind_of(args.qbits), fwd.view(), qv, did,
                                  static_cast<int>(ids.size()), args.k, args.decode_scale,
-                                 std::max(q.max_nnz, 1), dd, dl, s),
+                                 std::max(q.max_nnz, 1), r.d, r.l, s),
                "exact list launch");
-    download_results(ws, q.n, args.k, dd, dl, out_d, out_l);
+    download_results(ws, r, out_d, out_l);
 }
 
 }  // namespace nsp

@@ -137,7 +137,7 @@ protected:
 class Workspace : public Scratch {
 public:
     enum Slot : int {
-        kQIndptr, kQIdx, kQVal, kQCode, kOutD, kOutL, kSel, kBScore, kCounter, kStats,
+        kQuery, kQCode, kOut, kSel, kBScore, kStats,
         kCandD, kCandL, kHeapD, kHeapL, kQValG, kIds, kErr, kOrder, kSortKeys, kVisit, kQOrder,
         kNumSlots
     };
@@ -389,14 +389,18 @@ void exact_search(const ForwardDevice& fwd, const PostingsDevice* post, const Qu
 void exact_list_search(const ForwardDevice& fwd, const QueryBatch& q, const SeismicSearchArgs& args,
                        const std::vector<int32_t>& ids, float* out_d, int32_t* out_l);
 
-// Enqueues one SEISMIC search on `s`, its scratch drawn from `scratch`. With
-// `stats` null nothing on the host waits for the device (so the call can be
-// captured into a CUDA graph); else it waits and fills the kernel's time and
-// counters.
-void run_seismic(const ForwardDevice& fwd, const SeismicDevice& ix, int32_t n,
-                 const int32_t* d_indptr, const uint16_t* d_idx, const void* d_vals, int32_t qcap,
-                 const SeismicSearchArgs& args, const uint64_t* d_sel, float* d_out,
-                 int32_t* d_lab, cudaStream_t s, Scratch& scratch, SearchStats* stats);
+// Scratch slot kStats of a search: its counters, then the word the launch
+// claims queries from.
+constexpr size_t kControlBytes = (kStatCount + 1) * sizeof(unsigned long long);
+
+// Enqueues one SEISMIC search on `s`, its scratch drawn from `scratch`, and
+// returns the number of search launches. Nothing on the host waits for the
+// device, so the call can be captured into a CUDA graph; `timed` records the
+// calling thread's workspace events around the launches (not in a capture).
+int run_seismic(const ForwardDevice& fwd, const SeismicDevice& ix, int32_t n,
+                const int32_t* d_indptr, const uint16_t* d_idx, const void* d_vals, int32_t qcap,
+                const SeismicSearchArgs& args, const uint64_t* d_sel, float* d_out,
+                int32_t* d_lab, cudaStream_t s, Scratch& scratch, bool timed);
 
 // Grows the calling thread's workspace to what seismic_search of `n`
 // queries of up to `max_nnz` terms with `args` asks for, so a later search
@@ -409,7 +413,7 @@ void reserve_seismic_scratch(const ForwardDevice& fwd, const SeismicDevice& ix, 
 void seismic_search_device(const ForwardDevice& fwd, const SeismicDevice& ix, int32_t n,
                            const int32_t* d_indptr, const uint16_t* d_idx, const void* d_val,
                            int32_t max_nnz, const SeismicSearchArgs& args, const uint64_t* d_sel,
-                           float* d_out, int32_t* d_lab, cudaStream_t s, SearchStats* stats);
+                           float* d_out, int32_t* d_lab, cudaStream_t s);
 
 // Device buffers of a captured search step: the queries in CSR form (`n`
 // rows, room for `nnz_cap` entries; rows with terms ascending and unique) and

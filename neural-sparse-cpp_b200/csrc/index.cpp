@@ -649,7 +649,7 @@ void search_device(Index* index, int32_t n, const int32_t* d_indptr, const uint1
         d_sel = d;
     }
     nsp::seismic_search_device(st->vectors.dev, st->lists_dev, n, d_indptr, d_idx, vals, max_nnz,
-                               a, d_sel, d_out, d_lab, s, nullptr);
+                               a, d_sel, d_out, d_lab, s);
 }
 
 IndexSearchGraph::IndexSearchGraph(Index* index, int32_t n, int32_t nnz_cap, int32_t max_nnz,

@@ -202,7 +202,7 @@ extern "C" nsp_status_t nsp_index_search_device_noalloc(
             vals = codes;
         }
         nsp::run_seismic(st->vectors.dev, st->lists_dev, n, d_indptr, d_indices, vals,
-                         max_row_nnz, a, nullptr, d_distances, d_labels, stream, fixed, nullptr);
+                         max_row_nnz, a, nullptr, d_distances, d_labels, stream, fixed, false);
         return NSP_OK;
     } catch (const std::invalid_argument& e) {
         nsp::set_last_error(e.what());

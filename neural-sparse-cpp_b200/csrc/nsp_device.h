@@ -195,23 +195,76 @@ struct ExactLaunch {
     unsigned long long* stats;
 };
 
+// Driver queries whose answer never changes, remembered per thread for a few
+// keys (a lone query's call spent about 20 us in them).
+template <class Key, class Value, int kSlots>
+struct Memo {
+    Key key[kSlots] = {};
+    Value value[kSlots] = {};
+    bool used[kSlots] = {};
+    int next = 0;
+    const Value* find(const Key& k) const {
+        for (int i = 0; i < kSlots; ++i)
+            if (used[i] && key[i] == k) return &value[i];
+        return nullptr;
+    }
+    void put(const Key& k, const Value& v) {
+        key[next] = k;
+        value[next] = v;
+        used[next] = true;
+        next = (next + 1) % kSlots;
+    }
+};
+
+struct LaunchKey {
+    const void* f = nullptr;
+    int dev = 0, threads = 0, cluster = 0;
+    size_t smem = 0;
+    bool operator==(const LaunchKey& o) const {
+        return f == o.f && dev == o.dev && threads == o.threads && cluster == o.cluster &&
+               smem == o.smem;
+    }
+};
+
 // Lets kernel `f` use the device's whole opt-in shared memory (less its own
 // static shared memory, which counts against the same limit). Every call sets
 // the same value, so launches from several host threads cannot undo one
 // another's setting, as a per-launch size could between a set and a launch.
 template <class F>
 inline cudaError_t allow_opt_in_smem(F f) {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    static thread_local Memo<LaunchKey, bool, 16> done;
+    LaunchKey k;
+    k.f = reinterpret_cast<const void*>(f);
+    cudaError_t e = cudaGetDevice(&k.dev);
     if (e != cudaSuccess) return e;
+    if (done.find(k) != nullptr) return cudaSuccess;
     int v = 0;
-    e = cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    e = cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, k.dev);
     if (e != cudaSuccess) return e;
     cudaFuncAttributes fa{};
     e = cudaFuncGetAttributes(&fa, f);
     if (e != cudaSuccess) return e;
     const int dyn = v - static_cast<int>(fa.sharedSizeBytes);
-    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn > 0 ? dyn : 0);
+    e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn > 0 ? dyn : 0);
+    if (e == cudaSuccess) done.put(k, true);
+    return e;
+}
+
+// Resident CTAs of `f` per SM (0 on an error).
+template <class F>
+inline int resident_blocks(F f, int threads, size_t smem) {
+    static thread_local Memo<LaunchKey, int, 16> known;
+    LaunchKey k;
+    k.f = reinterpret_cast<const void*>(f);
+    k.threads = threads;
+    k.smem = smem;
+    if (cudaGetDevice(&k.dev) != cudaSuccess) return 0;
+    if (const int* b = known.find(k)) return *b;
+    int blocks = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, f, threads, smem) != cudaSuccess)
+        return 0;
+    known.put(k, blocks);
+    return blocks;
 }
 
 // Launchers (return cudaError_t of the launch). `sm_count` sizes persistent

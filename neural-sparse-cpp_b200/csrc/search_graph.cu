@@ -210,7 +210,7 @@ void SearchGraph::enqueue(cudaStream_t s) {
     }
     run_seismic(fwd_, ix_, n_, buf_.indptr, buf_.indices, vals, qcap_, args_,
                 own_->sel.size() > 0 ? own_->sel.data() : nullptr, buf_.distances, buf_.labels, s,
-                own_->scratch, nullptr);
+                own_->scratch, false);
 }
 
 void SearchGraph::launch(cudaStream_t s) {

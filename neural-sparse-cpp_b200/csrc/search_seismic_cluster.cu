@@ -717,18 +717,27 @@ cudaError_t launch_typed(const SeismicLaunch& a, int warps, int blocks, size_t s
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    if (a.cluster > 8) {  // past the portable size
-        e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (e != cudaSuccess) {
-            (void)cudaGetLastError();
-            return cudaSuccess;
-        }
+    static thread_local Memo<LaunchKey, bool, 16> known;  // whether it can be placed
+    LaunchKey k;
+    k.f = reinterpret_cast<const void*>(f);
+    k.threads = warps * 32;
+    k.cluster = a.cluster;
+    k.smem = smem;
+    e = cudaGetDevice(&k.dev);
+    if (e != cudaSuccess) return e;
+    const bool* fits = known.find(k);
+    if (fits == nullptr) {
+        bool ok = true;
+        if (a.cluster > 8)  // past the portable size
+            ok = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                 cudaSuccess;
+        int clusters = 0;
+        ok = ok && cudaOccupancyMaxActiveClusters(&clusters, f, &cfg) == cudaSuccess && clusters > 0;
+        if (!ok) (void)cudaGetLastError();
+        known.put(k, ok);
+        fits = known.find(k);
     }
-    int fits = 0;
-    if (cudaOccupancyMaxActiveClusters(&fits, f, &cfg) != cudaSuccess || fits <= 0) {
-        (void)cudaGetLastError();
-        return cudaSuccess;
-    }
+    if (!*fits) return cudaSuccess;
     placed = true;
     return cudaLaunchKernelEx(&cfg, f, a);
 }

@@ -421,11 +421,7 @@ template <typename V, typename TE, int kG>
 int max_blocks_cta_g(int threads, size_t smem) {
     if (allow_opt_in_smem(seismic_cta_kernel<V, TE, kG>) != cudaSuccess)
         return 0;
-    int blocks = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, seismic_cta_kernel<V, TE, kG>,
-                                                      threads, smem) != cudaSuccess)
-        return 0;
-    return blocks;
+    return resident_blocks(seismic_cta_kernel<V, TE, kG>, threads, smem);
 }
 
 template <typename V, typename TE>
