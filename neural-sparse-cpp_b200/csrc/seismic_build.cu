@@ -209,7 +209,6 @@ struct AssignArgs {
     int32_t* work;          // list counter
     // per-CTA scratch
     int32_t* tcnt;          // [dim] per CTA, zero between lists
-    int32_t* tstart;        // [dim] per CTA
     int32_t* tcur;          // [dim] per CTA
     int2* trun;             // [dim] per CTA: (start, count) of the term's centroid
                             // entries, count zero between lists
@@ -222,7 +221,14 @@ struct AssignArgs {
     int64_t max_kept;
     int32_t max_nc;
     int32_t sims_in_smem;  // 1: the similarity rows are in dynamic shared memory
+    // fp32: after them, rows of the list's terms that most centroids hold, a
+    // value per centroid (max_nc, a multiple of 4, floats each)
+    int32_t dense_rows;
 };
+
+// A term's centroid run as (start, count | (dense row + 1) << kDenseShift).
+constexpr int kDenseShift = 20;  // counts are at most 65,536 centroids
+constexpr int kMaxDenseRows = 64;
 
 // Similarity accumulators: fp32 for fp32 values; int for uint8 codes (at
 // most 400 products of two codes below 2^16 each, exact), int64 for uint16.
@@ -230,26 +236,40 @@ template <int ESZ>
 using assign_acc_t = typename std::conditional<
     ESZ == 4, float, typename std::conditional<ESZ == 1, int, long long>::type>::type;
 
-// One centroid entry of a term's run: the centroid and its value.
 template <int ESZ>
-__device__ __forceinline__ void centroid_entry(const uint16_t* ccl, const uint8_t* cw, int32_t k,
-                                               int32_t& c, assign_acc_t<ESZ>& w) {
-    c = ccl[k];
-    if constexpr (ESZ == 4) w = reinterpret_cast<const float*>(cw)[k];
-    else if constexpr (ESZ == 2) w = reinterpret_cast<const uint16_t*>(cw)[k];
-    else w = cw[k];
+using assign_val_t = typename std::conditional<
+    ESZ == 4, float, typename std::conditional<ESZ == 1, uint8_t, uint16_t>::type>::type;
+
+__device__ __forceinline__ void add_product(float* sims, int32_t c, float dv, float w) {
+    sims[c] = __fadd_rn(sims[c], __fmul_rn(dv, w));
+}
+template <class T>
+__device__ __forceinline__ void add_product(T* sims, int32_t c, T dv, T w) {
+    sims[c] += dv * w;
 }
 
-template <int ESZ>
-__device__ __forceinline__ void add_product(assign_acc_t<ESZ>* sims, int32_t c,
-                                            assign_acc_t<ESZ> dv, assign_acc_t<ESZ> w) {
-    if constexpr (ESZ == 4) sims[c] = __fadd_rn(sims[c], __fmul_rn(dv, w));
-    else sims[c] += dv * w;
+// sims[c] += dv * row[c] for every centroid (n4 a multiple of 4).
+__device__ __forceinline__ void apply_dense(float* sims, const float* row, float dv, int32_t n4,
+                                            int lane) {
+    const float4* w4 = reinterpret_cast<const float4*>(row);
+    float4* s4 = reinterpret_cast<float4*>(sims);
+    for (int32_t c = lane; c < n4 / 4; c += 32) {
+        const float4 w = w4[c];
+        float4 x = s4[c];
+        x.x = __fadd_rn(x.x, __fmul_rn(dv, w.x));
+        x.y = __fadd_rn(x.y, __fmul_rn(dv, w.y));
+        x.z = __fadd_rn(x.z, __fmul_rn(dv, w.z));
+        x.w = __fadd_rn(x.w, __fmul_rn(dv, w.w));
+        s4[c] = x;
+    }
 }
+template <class T>
+__device__ __forceinline__ void apply_dense(T*, const float*, T, int32_t, int) {}
 
 template <int ESZ>
 __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
     using acc_t = assign_acc_t<ESZ>;
+    using val_t = assign_val_t<ESZ>;
     // centroid entries of one term in flight per lane: a term's run is
     // loaded kChunks * 32 entries at a time, the next hit term's first
     // chunk while the current one is applied
@@ -257,17 +277,18 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
     __shared__ int32_t s_list;
     __shared__ int32_t s_touched;
     __shared__ int32_t s_total;
+    __shared__ int32_t s_dense;
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int wpb = blockDim.x >> 5;
     const int dim = a.f.dim;
     int32_t* tcnt = a.tcnt + static_cast<size_t>(blockIdx.x) * dim;
-    int32_t* tstart = a.tstart + static_cast<size_t>(blockIdx.x) * dim;
     int32_t* tcur = a.tcur + static_cast<size_t>(blockIdx.x) * dim;
     int2* trun = a.trun + static_cast<size_t>(blockIdx.x) * dim;
     int32_t* touched = a.touched + static_cast<size_t>(blockIdx.x) * a.max_centroid_entries;
     uint16_t* ccl = a.ccl + static_cast<size_t>(blockIdx.x) * a.max_centroid_entries;
-    uint8_t* cw = a.cw + static_cast<size_t>(blockIdx.x) * a.max_centroid_entries * ESZ;
+    val_t* vals = reinterpret_cast<val_t*>(
+        a.cw + static_cast<size_t>(blockIdx.x) * a.max_centroid_entries * ESZ);
     uint8_t* isc = a.is_centroid + static_cast<size_t>(blockIdx.x) * a.max_kept;
     // each warp's row of similarities: shared memory when the launch gave
     // room for it (the read-modify-writes of one doc are serial), else global
@@ -275,7 +296,20 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
     acc_t* sims = a.sims_in_smem ? reinterpret_cast<acc_t*>(dyn) + static_cast<size_t>(warp) * a.max_nc
                                  : static_cast<acc_t*>(a.sims) +
                                        static_cast<size_t>(blockIdx.x * wpb + warp) * a.max_nc;
-    const uint8_t* fval = static_cast<const uint8_t*>(a.f.val);
+    // Bound by shared memory: a product is a read-modify-write of its
+    // similarity, and a warp's 32 scattered ones conflict in the banks. A term
+    // that at least 30% of the list's centroids hold is therefore applied as a
+    // dense row of shared memory, four centroids per lane and no conflicts
+    // (below that share the row's zero products cost more than the conflicts);
+    // centroids without the term add a zero product, which leaves a sum as it
+    // is while the doc's value is finite. Staging the other terms' runs in
+    // shared memory as well, 32 terms at a time, was slower: the stage is more
+    // of the same traffic (80,000 docs, lambda 4000, beta 400, assignment: 89
+    // ms without rows, 80 with them and with four entries in flight in the
+    // indexing below, 101 with the stage).
+    constexpr bool kDense = ESZ == 4;
+    float* rows = reinterpret_cast<float*>(dyn) + static_cast<size_t>(wpb) * a.max_nc;
+    const val_t* fval = static_cast<const val_t*>(a.f.val);
 
     for (;;) {
         if (threadIdx.x == 0) s_list = atomicAdd(a.work, 1);
@@ -297,9 +331,13 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
         if (threadIdx.x == 0) {
             s_touched = 0;
             s_total = 0;
+            s_dense = 0;
         }
         __syncthreads();
-        for (int32_t c = threadIdx.x; c < nc; c += blockDim.x) isc[cp[c]] = 1;
+        for (int32_t c = threadIdx.x; c < nc; c += blockDim.x) {
+            isc[cp[c]] = 1;
+            a.out_key[kb + cp[c]] = static_cast<uint32_t>(c) * 2u;  // its own cluster, placed first
+        }
         // index the centroid entries by term: count, ranges, scatter
         for (int32_t c = warp; c < nc; c += wpb) {
             const int32_t doc = a.kept[kb + cp[c]];
@@ -316,36 +354,55 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
             const int32_t term = touched[i];
             const int32_t cnt = tcnt[term];
             const int32_t st = atomicAdd(&s_total, cnt);
-            tstart[term] = st;
-            tcur[term] = 0;
-            trun[term] = make_int2(st, cnt);
+            tcur[term] = st;
+            int32_t row = 0;
+            if (kDense && a.dense_rows > 0 && 10ll * cnt >= 3ll * nc) {
+                row = atomicAdd(&s_dense, 1) + 1;
+                if (row > a.dense_rows) row = 0;
+            }
+            trun[term] = make_int2(st, cnt | (row << kDenseShift));
         }
         __syncthreads();
+        const int32_t nc4 = (nc + 3) & ~3;
+        if constexpr (kDense) {
+            const int32_t cells = min(s_dense, a.dense_rows) * nc4;
+            for (int32_t i = threadIdx.x; i < cells; i += blockDim.x) rows[i] = 0.0f;
+            __syncthreads();
+        }
         for (int32_t c = warp; c < nc; c += wpb) {
             const int32_t doc = a.kept[kb + cp[c]];
             const uint2 ri = a.f.rowinfo[doc];
             const int64_t rb = static_cast<int64_t>(ri.x) * nsp::kRowAlign;
-            for (uint32_t e = lane; e < ri.y; e += 32) {
-                const int32_t term = a.f.idx[rb + e];
-                const int32_t pos = tstart[term] + atomicAdd(tcur + term, 1);
-                ccl[pos] = static_cast<uint16_t>(c);
-                for (int b = 0; b < ESZ; ++b) cw[static_cast<size_t>(pos) * ESZ + b] = fval[(rb + e) * ESZ + b];
+            for (uint32_t e0 = 0; e0 < ri.y; e0 += 128) {  // four entries in flight per lane
+                int32_t pos[4], row[4];
+                val_t w[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const uint32_t e = e0 + u * 32 + lane;
+                    pos[u] = -1;
+                    if (e < ri.y) {
+                        const int32_t term = a.f.idx[rb + e];
+                        w[u] = fval[rb + e];
+                        pos[u] = atomicAdd(tcur + term, 1);
+                        if constexpr (kDense) row[u] = trun[term].y >> kDenseShift;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if (pos[u] < 0) continue;
+                    ccl[pos[u]] = static_cast<uint16_t>(c);
+                    vals[pos[u]] = w[u];
+                    if constexpr (kDense)
+                        if (row[u] > 0) rows[(row[u] - 1) * nc4 + c] = w[u];
+                }
             }
         }
         __syncthreads();
         // assign every non-centroid doc, one warp per doc
         for (int32_t p = warp; p < n; p += wpb) {
-            if (isc[p]) {
-                // centroid: its own cluster, placed first
-                if (lane == 0) {
-                    int32_t c = 0;
-                    while (cp[c] != p) ++c;
-                    a.out_key[kb + p] = static_cast<uint32_t>(c) * 2u;
-                }
-                continue;
-            }
+            if (isc[p]) continue;
             const int32_t doc = a.kept[kb + p];
-            for (int32_t c = lane; c < nc; c += 32) sims[c] = 0;
+            for (int32_t c = lane; c < nc4; c += 32) sims[c] = 0;
             __syncwarp();
             const uint2 ri = a.f.rowinfo[doc];
             const int64_t rb = static_cast<int64_t>(ri.x) * nsp::kRowAlign;
@@ -355,9 +412,7 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
                 acc_t v = 0;
                 if (e < ri.y) {
                     run = trun[a.f.idx[rb + e]];
-                    if constexpr (ESZ == 4) v = reinterpret_cast<const float*>(fval)[rb + e];
-                    else if constexpr (ESZ == 2) v = reinterpret_cast<const uint16_t*>(fval)[rb + e];
-                    else v = fval[rb + e];
+                    v = fval[rb + e];
                 }
                 // doc terms in order (kmeans_utils.cpp:134-145); a term's
                 // centroids are distinct, so its products commute, and the
@@ -366,20 +421,30 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
                 unsigned m = __ballot_sync(kFull, run.y > 0);
                 int32_t nc_[kChunks];
                 acc_t nw[kChunks];
-                int32_t s0 = 0, cnt = 0;
+                int32_t s0 = 0, cnt = 0, row = 0;
                 acc_t dv = 0;
-                if (m) {
-                    const int src = __ffs(m) - 1;
+                // the hit term of lane src: its value, and its dense row or
+                // the first entries of its run
+                auto fetch = [&](int src) {
                     s0 = __shfl_sync(kFull, run.x, src);
                     cnt = __shfl_sync(kFull, run.y, src);
                     dv = __shfl_sync(kFull, v, src);
+                    row = 0;
+                    if constexpr (kDense) {
+                        row = isfinite(dv) ? cnt >> kDenseShift : 0;
+                        cnt &= (1 << kDenseShift) - 1;
+                    }
 #pragma unroll
                     for (int j = 0; j < kChunks; ++j) {
                         const int32_t k = j * 32 + lane;
                         nc_[j] = -1;
-                        if (k < cnt) centroid_entry<ESZ>(ccl, cw, s0 + k, nc_[j], nw[j]);
+                        if (row == 0 && k < cnt) {
+                            nc_[j] = ccl[s0 + k];
+                            nw[j] = vals[s0 + k];
+                        }
                     }
-                }
+                };
+                if (m) fetch(__ffs(m) - 1);
                 while (m) {
                     m &= m - 1;
                     int32_t cc[kChunks];
@@ -389,33 +454,30 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
                         cc[j] = nc_[j];
                         cwv[j] = nw[j];
                     }
-                    const int32_t cs0 = s0, ccnt = cnt;
+                    const int32_t cs0 = s0, ccnt = cnt, crow = row;
                     const acc_t cdv = dv;
-                    if (m) {
-                        const int src = __ffs(m) - 1;
-                        s0 = __shfl_sync(kFull, run.x, src);
-                        cnt = __shfl_sync(kFull, run.y, src);
-                        dv = __shfl_sync(kFull, v, src);
-#pragma unroll
-                        for (int j = 0; j < kChunks; ++j) {
-                            const int32_t k = j * 32 + lane;
-                            nc_[j] = -1;
-                            if (k < cnt) centroid_entry<ESZ>(ccl, cw, s0 + k, nc_[j], nw[j]);
-                        }
+                    if (m) fetch(__ffs(m) - 1);
+                    if (kDense && crow > 0) {
+                        apply_dense(sims, rows + (crow - 1) * nc4, cdv, nc4, lane);
+                        __syncwarp();
+                        continue;
                     }
 #pragma unroll
                     for (int j = 0; j < kChunks; ++j)
-                        if (cc[j] >= 0) add_product<ESZ>(sims, cc[j], cdv, cwv[j]);
+                        if (cc[j] >= 0) add_product(sims, cc[j], cdv, cwv[j]);
                     for (int32_t k0 = kChunks * 32; k0 < ccnt; k0 += kChunks * 32) {
 #pragma unroll
                         for (int j = 0; j < kChunks; ++j) {
                             const int32_t k = k0 + j * 32 + lane;
                             cc[j] = -1;
-                            if (k < ccnt) centroid_entry<ESZ>(ccl, cw, cs0 + k, cc[j], cwv[j]);
+                            if (k < ccnt) {
+                                cc[j] = ccl[cs0 + k];
+                                cwv[j] = vals[cs0 + k];
+                            }
                         }
 #pragma unroll
                         for (int j = 0; j < kChunks; ++j)
-                            if (cc[j] >= 0) add_product<ESZ>(sims, cc[j], cdv, cwv[j]);
+                            if (cc[j] >= 0) add_product(sims, cc[j], cdv, cwv[j]);
                     }
                     __syncwarp();
                 }
@@ -646,10 +708,18 @@ void build_typed(SeismicState& st, int dim, const SeismicClusterParameters& p) {
         const int64_t max_ce = std::max<int64_t>(1, static_cast<int64_t>(max_nc) * max_row);
         const int wpb = 32;
         const size_t acc_bytes = sizeof(assign_acc_t<ESZ>);
-        const size_t sims_smem = static_cast<size_t>(wpb) * std::max(max_nc, 1) * acc_bytes;
+        const int32_t nc_row = (std::max(max_nc, 1) + 3) & ~3;
+        const size_t sims_smem = static_cast<size_t>(wpb) * nc_row * acc_bytes;
         const bool sims_in_smem = sims_smem <= 160u * 1024u;
-        const size_t smem = sims_in_smem ? sims_smem : 0;
-        if (sims_in_smem) cuda_check(nsp::allow_opt_in_smem(assign_kernel<ESZ>), "assign smem");
+        // dense rows in what is left of 224 KB
+        int32_t dense_rows = 0;
+        if (ESZ == 4 && sims_in_smem)
+            dense_rows = static_cast<int32_t>(std::min<size_t>(
+                kMaxDenseRows, (224u * 1024u - sims_smem) / (static_cast<size_t>(nc_row) * 4)));
+        const size_t smem =
+            sims_in_smem ? sims_smem + static_cast<size_t>(dense_rows) * nc_row * 4 : 0;
+        if (sims_in_smem)
+            cuda_check(nsp::allow_opt_in_smem(assign_kernel<ESZ>), "assign smem");
         // one CTA of 32 warps per SM: as many warps as four CTAs of 8 hide
         // the memory round trips with, and a quarter of the per-CTA term
         // tables (trun, tcnt, ...), which then stay in L2 (8.8M SQ docs:
@@ -670,11 +740,11 @@ void build_typed(SeismicState& st, int dim, const SeismicClusterParameters& p) {
         a.out_key = akey;
         a.max_centroid_entries = max_ce;
         a.max_kept = std::max<int64_t>(max_kept, 1);
-        a.max_nc = std::max(max_nc, 1);
+        a.max_nc = nc_row;
+        a.dense_rows = dense_rows;
         a.sims_in_smem = sims_in_smem ? 1 : 0;
         a.work = arena.take<int32_t>(1);
         a.tcnt = arena.take<int32_t>(ctas * dim);
-        a.tstart = arena.take<int32_t>(ctas * dim);
         a.tcur = arena.take<int32_t>(ctas * dim);
         a.trun = arena.take<int2>(ctas * dim);
         a.touched = arena.take<int32_t>(ctas * max_ce);
