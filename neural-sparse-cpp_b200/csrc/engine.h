@@ -320,7 +320,8 @@ struct KernelChoice {
 // CTAs per query the engine gives a launch of `n_queries` queries: the most
 // of 1, 2, 4, 8 that still gives every query its own SMs (n * c <= SM count),
 // so a launch of few queries spreads each over a thread-block cluster; large
-// launches keep one CTA per query.
+// launches keep one CTA per query. Launches of up to four queries get 16: a
+// cluster of 16 takes most of a GPC, so only a few run at once.
 int auto_cluster(int n_queries);
 
 struct SeismicSearchArgs {
@@ -337,7 +338,7 @@ struct SeismicSearchArgs {
                               // 2-5 one CTA per query with 1, 2, 4, 8 lanes per doc
     int stage_bytes = 0;      // staged: bytes per stage buffer (0 = default)
     int batch_docs = 0;       // variants 2-5: candidate docs per batch (0 = default)
-    int cluster = 0;          // variants 2-5: CTAs per query (0 = engine's choice, 1, 2, 4, 8)
+    int cluster = 0;          // variants 2-5: CTAs per query (0 = engine's choice up to 16, 1, 2, 4, 8)
     // variants 2-5: one device doc bitmap per query (a null entry admits every
     // doc), in device memory; replaces the launch-wide selector
     const uint64_t* const* d_sel_q = nullptr;

@@ -33,7 +33,7 @@
 // Measured, all summaries of a build: fp32, 80,000 docs, lambda 4000 (1.2G
 // entries in 3.7M blocks): 0.79 s when the entries were
 // sorted by term and the maxima by value (about ten passes over global
-// memory), 0.13 s now, 0.06 s of it in these kernels; SEISMIC-SQ 8-bit,
+// memory), 0.08 s now, 0.06 s of it in these kernels; SEISMIC-SQ 8-bit,
 // 200,000 docs, lambda 6000 (3.2G entries): 0.33 s with a hash table per block
 // and two passes, 0.15 s now, 0.05 s in these kernels.
 #include <cuda_runtime.h>
