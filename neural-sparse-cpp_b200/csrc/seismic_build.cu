@@ -298,14 +298,15 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
                                        static_cast<size_t>(blockIdx.x * wpb + warp) * a.max_nc;
     // Bound by shared memory: a product is a read-modify-write of its
     // similarity, and a warp's 32 scattered ones conflict in the banks. A term
-    // that at least 30% of the list's centroids hold is therefore applied as a
+    // that at least 40% of the list's centroids hold is therefore applied as a
     // dense row of shared memory, four centroids per lane and no conflicts
-    // (below that share the row's zero products cost more than the conflicts);
+    // (below that share the row's zero products cost more than the conflicts:
+    // with 20% the case below takes 84 ms, with 30% 80);
     // centroids without the term add a zero product, which leaves a sum as it
     // is while the doc's value is finite. Staging the other terms' runs in
     // shared memory as well, 32 terms at a time, was slower: the stage is more
     // of the same traffic (80,000 docs, lambda 4000, beta 400, assignment: 89
-    // ms without rows, 80 with them and with four entries in flight in the
+    // ms without rows, 78 with them and with four entries in flight in the
     // indexing below, 101 with the stage).
     constexpr bool kDense = ESZ == 4;
     float* rows = reinterpret_cast<float*>(dyn) + static_cast<size_t>(wpb) * a.max_nc;
@@ -356,7 +357,7 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
             const int32_t st = atomicAdd(&s_total, cnt);
             tcur[term] = st;
             int32_t row = 0;
-            if (kDense && a.dense_rows > 0 && 10ll * cnt >= 3ll * nc) {
+            if (kDense && a.dense_rows > 0 && 10ll * cnt >= 4ll * nc) {
                 row = atomicAdd(&s_dense, 1) + 1;
                 if (row > a.dense_rows) row = 0;
             }
