@@ -21,7 +21,9 @@
 //
 // Control words: rank 0 writes a batch's size into every CTA before a cluster
 // barrier (kNextLists: summaries of the next lists; kQueryDone), so all CTAs
-// pass the same barriers in the same order and nothing spins.
+// pass the same barriers in the same order and nothing spins. Between two
+// writes of one word lies at least one barrier that its readers arrive at
+// after their read, for queries without lists too.
 //
 // Measured, one query per call (whole calls): fp32, 100,000 docs 431 -> 275 us,
 // SQ, 3M docs 689 -> 385 us, against the same cluster with rank 0 doing 2-4
@@ -648,6 +650,10 @@ __global__ void __launch_bounds__(1024, 1) seismic_cluster_kernel(SeismicLaunch 
                 }
             }
         }
+        // A query of no lists passed none of the barriers above: without this
+        // one the leader could write the next query's number over the one
+        // that another CTA's threads are still about to read.
+        if (ncut == 0) cluster_sync();
         // results, padded with (-1.0, -1); SQ scores decoded
         // (seismic_scalar_quantized_index.cpp:345-355)
         if (rank == 0 && warp == 0) {
