@@ -13,11 +13,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <climits>
 #include <cstdint>
 #include <vector>
 
 #include "engine.h"
+#include "postings_plan.h"
 #include "scan.h"
 
 namespace nsp {
@@ -124,12 +124,13 @@ __global__ void dense_rows_kernel(const int32_t* terms, int n_dense, const int32
                                   const int32_t* doc, const float* val, int C, float* dense) {
     const int j = blockIdx.y;
     const int t = terms[j];
-    for (int32_t p = tstart[t] + static_cast<int32_t>(blockIdx.x * blockDim.x + threadIdx.x);
-         p < tstart[t + 1]; p += static_cast<int32_t>(gridDim.x * blockDim.x)) {
-        const int32_t d = doc[p];
-        const int32_t c = d / C;
-        dense[(static_cast<size_t>(c) * n_dense + j) * C + (d - c * C)] = val[p];
-    }
+    const int64_t first = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    each_posting(tstart[t], tstart[t + 1], first, static_cast<int64_t>(gridDim.x) * blockDim.x,
+                 [&](int32_t p) {
+                     const int32_t d = doc[p];
+                     const int32_t c = d / C;
+                     dense[(static_cast<size_t>(c) * n_dense + j) * C + (d - c * C)] = val[p];
+                 });
 }
 
 int grid_for(int64_t work, int per_block) {
@@ -170,7 +171,7 @@ void PostingsDevice::build(const ForwardDevice& fwd, int chunk_docs) {
     cuda_check(cudaMemcpyAsync(&unsorted, flag, sizeof(int), cudaMemcpyDeviceToHost, s),
                "D2H");
     cuda_check(cudaStreamSynchronize(s), "sync");
-    if (unsorted != 0 || nnz >= INT_MAX) return;  // the tile kernel serves this index
+    if (unsorted != 0 || nnz > kMaxPostings) return;  // the tile kernel serves this index
 
     n_chunks_ = (n + chunk_docs - 1) / chunk_docs;
     const int dim = f.dim;

@@ -26,6 +26,7 @@
 #include <cstdint>
 
 #include "nsp_device.h"
+#include "postings_plan.h"
 
 namespace nsp {
 namespace {
@@ -522,6 +523,8 @@ __global__ void __launch_bounds__(kTThreads) exact_taat_kernel(ExactLaunch a) {
     const int stride = P.n_chunks + 1;
     constexpr int B = kTThreads;
     constexpr int kAhead = 4;  // postings per thread loaded a term ahead
+    // the furthest position computed past a run's first, below
+    static_assert((1 + kAhead + 3) * B <= kPostingsAhead, "postings end below 2^31");
     unsigned long long postings = 0, dense_docs = 0;
     for (int w0 = 0; w0 < qn; w0 += kTermWin) {
         const int wn = min(kTermWin, qn - w0);
