@@ -634,9 +634,7 @@ bool assign_u8(const FwdView& f, const AssignLists& lists, const std::vector<int
     a.max_kept = max_kept;
     a.ld = ld;
     const size_t smem = smem_layout(hot_bytes, words).total;
-    cuda_check(cudaFuncSetAttribute(assign_u8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(smem)),
-               "cudaFuncSetAttribute");
+    cuda_check(allow_opt_in_smem(assign_u8_kernel), "assign shared memory");
     assign_u8_kernel<<<ctas, kThreads, smem, s>>>(a);
     cuda_check(cudaGetLastError(), "assign_u8_kernel");
     int32_t err = 0;

@@ -1163,9 +1163,7 @@ void summarize_typed(const FwdView& f, const BlockSet& blocks, float alpha, cons
             p.smem_vals = false;
             p.smem = sum_layout(p.cap, p.sel, w, false).total;
         }
-        cuda_check(cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(p.smem)),
-                   "cudaFuncSetAttribute");
+        cuda_check(allow_opt_in_smem(p.kernel), "summary shared memory");
         int per_sm = 0;
         cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p.kernel, p.warps * 32,
                                                                  p.smem),
