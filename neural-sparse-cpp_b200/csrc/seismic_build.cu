@@ -230,11 +230,13 @@ struct AssignArgs {
 constexpr int kDenseShift = 20;  // counts are at most 65,536 centroids
 constexpr int kMaxDenseRows = 64;
 
-// Similarity accumulators: fp32 for fp32 values; int for uint8 codes (at
-// most 400 products of two codes below 2^16 each, exact), int64 for uint16.
-template <int ESZ>
+// Similarity accumulators: fp32 for fp32 values; for codes int64, or int for
+// uint8 codes of rows without repeated terms (a product per entry of the
+// doc's row).
+template <int ESZ, bool kRepeats>
 using assign_acc_t = typename std::conditional<
-    ESZ == 4, float, typename std::conditional<ESZ == 1, int, long long>::type>::type;
+    ESZ == 4, float,
+    typename std::conditional<ESZ == 1 && !kRepeats, int, long long>::type>::type;
 
 template <int ESZ>
 using assign_val_t = typename std::conditional<
@@ -246,6 +248,19 @@ __device__ __forceinline__ void add_product(float* sims, int32_t c, float dv, fl
 template <class T>
 __device__ __forceinline__ void add_product(T* sims, int32_t c, T dv, T w) {
     sims[c] += dv * w;
+}
+
+// Lane by lane the products of 32 entries of a term's run (c < 0: none), where
+// a centroid may hold several: its entries are added one after another, in
+// lane order. By a whole warp.
+template <class T>
+__device__ __forceinline__ void add_products_in_turn(T* sims, int32_t c, T dv, T w, int lane) {
+    const unsigned peers = __match_any_sync(kFull, c);
+    const int turn = c < 0 ? -1 : __popc(peers & ((1u << lane) - 1u));
+    for (int r = 0; __any_sync(kFull, turn >= r); ++r) {
+        if (turn == r) add_product(sims, c, dv, w);
+        __syncwarp();
+    }
 }
 
 // sims[c] += dv * row[c] for every centroid (n4 a multiple of 4).
@@ -266,9 +281,14 @@ __device__ __forceinline__ void apply_dense(float* sims, const float* row, float
 template <class T>
 __device__ __forceinline__ void apply_dense(T*, const float*, T, int32_t, int) {}
 
-template <int ESZ>
+// kRepeats: some row repeats a term. A centroid then has several entries in
+// one term's run, which the reference adds in the centroid's order
+// (kmeans_utils.cpp:40-97): one warp indexes the centroids in order, so a run
+// lists them as they come, and entries of one centroid take turns. Other
+// indexes have distinct centroids in a run, whose products commute.
+template <int ESZ, bool kRepeats>
 __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
-    using acc_t = assign_acc_t<ESZ>;
+    using acc_t = assign_acc_t<ESZ, kRepeats>;
     using val_t = assign_val_t<ESZ>;
     // centroid entries of one term in flight per lane: a term's run is
     // loaded kChunks * 32 entries at a time, the next hit term's first
@@ -308,7 +328,7 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
     // of the same traffic (80,000 docs, lambda 4000, beta 400, assignment: 89
     // ms without rows, 78 with them and with four entries in flight in the
     // indexing below, 101 with the stage).
-    constexpr bool kDense = ESZ == 4;
+    constexpr bool kDense = ESZ == 4 && !kRepeats;  // (a row's cell holds one entry)
     float* rows = reinterpret_cast<float*>(dyn) + static_cast<size_t>(wpb) * a.max_nc;
     const val_t* fval = static_cast<const val_t*>(a.f.val);
 
@@ -370,7 +390,28 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
             for (int32_t i = threadIdx.x; i < cells; i += blockDim.x) rows[i] = 0.0f;
             __syncthreads();
         }
-        for (int32_t c = warp; c < nc; c += wpb) {
+        if constexpr (kRepeats) {
+            for (int32_t c = 0; c < nc && warp == 0; ++c) {
+                const int32_t doc = a.kept[kb + cp[c]];
+                const uint2 ri = a.f.rowinfo[doc];
+                const int64_t rb = static_cast<int64_t>(ri.x) * nsp::kRowAlign;
+                for (uint32_t e0 = 0; e0 < ri.y; e0 += 32) {
+                    const uint32_t e = e0 + lane;
+                    const int32_t term = e < ri.y ? a.f.idx[rb + e] : -1;
+                    const unsigned peers = __match_any_sync(kFull, term);
+                    const int rank = __popc(peers & ((1u << lane) - 1u));
+                    const int32_t at = term >= 0 ? tcur[term] : 0;
+                    __syncwarp();
+                    if (term >= 0) {
+                        ccl[at + rank] = static_cast<uint16_t>(c);
+                        vals[at + rank] = fval[rb + e];
+                        if (rank == 0) tcur[term] = at + __popc(peers);
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+        for (int32_t c = warp; c < nc && !kRepeats; c += wpb) {
             const int32_t doc = a.kept[kb + cp[c]];
             const uint2 ri = a.f.rowinfo[doc];
             const int64_t rb = static_cast<int64_t>(ri.x) * nsp::kRowAlign;
@@ -464,8 +505,12 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
                         continue;
                     }
 #pragma unroll
-                    for (int j = 0; j < kChunks; ++j)
-                        if (cc[j] >= 0) add_product(sims, cc[j], cdv, cwv[j]);
+                    for (int j = 0; j < kChunks; ++j) {
+                        if constexpr (kRepeats)
+                            add_products_in_turn(sims, cc[j], cdv, cwv[j], lane);
+                        else if (cc[j] >= 0)
+                            add_product(sims, cc[j], cdv, cwv[j]);
+                    }
                     for (int32_t k0 = kChunks * 32; k0 < ccnt; k0 += kChunks * 32) {
 #pragma unroll
                         for (int j = 0; j < kChunks; ++j) {
@@ -477,8 +522,12 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
                             }
                         }
 #pragma unroll
-                        for (int j = 0; j < kChunks; ++j)
-                            if (cc[j] >= 0) add_product(sims, cc[j], cdv, cwv[j]);
+                        for (int j = 0; j < kChunks; ++j) {
+                            if constexpr (kRepeats)
+                                add_products_in_turn(sims, cc[j], cdv, cwv[j], lane);
+                            else if (cc[j] >= 0)
+                                add_product(sims, cc[j], cdv, cwv[j]);
+                        }
                     }
                     __syncwarp();
                 }
@@ -511,6 +560,33 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
             trun[touched[i]] = make_int2(0, 0);
         }
         __syncthreads();
+    }
+}
+
+// *repeats = 1 when some row holds a term twice: a warp per row, a bitmap of
+// the terms seen for the rows that are not strictly ascending.
+constexpr int kSeenWarps = 4;
+__global__ void __launch_bounds__(kSeenWarps * 32) repeats_kernel(nsp::FwdView f, int* repeats) {
+    __shared__ uint32_t seen[kSeenWarps][65536 / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i = lane; i < 65536 / 32; i += 32) seen[warp][i] = 0u;
+    __syncwarp();
+    for (int64_t d = static_cast<int64_t>(blockIdx.x) * kSeenWarps + warp; d < f.n_docs;
+         d += static_cast<int64_t>(gridDim.x) * kSeenWarps) {
+        const uint2 ri = __ldg(f.rowinfo + d);
+        const uint16_t* ip = f.idx + static_cast<size_t>(ri.x) * nsp::kRowAlign;
+        bool bad = false;
+        for (uint32_t e = 1 + lane; e < ri.y; e += 32) bad |= __ldg(ip + e - 1) >= __ldg(ip + e);
+        if (!__any_sync(kFull, bad)) continue;
+        bool twice = false;
+        for (uint32_t e = lane; e < ri.y; e += 32) {
+            const uint32_t t = __ldg(ip + e), bit = 1u << (t & 31);
+            twice |= (atomicOr(&seen[warp][t >> 5], bit) & bit) != 0u;
+        }
+        if (__any_sync(kFull, twice) && lane == 0) *repeats = 1;
+        __syncwarp();
+        for (uint32_t e = lane; e < ri.y; e += 32) seen[warp][__ldg(ip + e) >> 5] = 0u;
+        __syncwarp();
     }
 }
 
@@ -595,6 +671,66 @@ struct PhaseClock {
         t = now;
     }
 };
+
+// Assignment by assign_kernel: any values, any rows.
+template <int ESZ, bool kRepeats>
+void assign_general(const nsp::FwdView& f, const nsp::AssignLists& l, uint32_t* out_key,
+                    cudaStream_t s, nsp::Arena& scratch) {
+    const int dim = f.dim;
+    const int64_t max_ce = std::max<int64_t>(1, static_cast<int64_t>(l.max_nc) * l.max_row);
+    const int wpb = 32;
+    const size_t acc_bytes = sizeof(assign_acc_t<ESZ, kRepeats>);
+    const int32_t nc_row = (std::max(l.max_nc, 1) + 3) & ~3;
+    const size_t sims_smem = static_cast<size_t>(wpb) * nc_row * acc_bytes;
+    const bool sims_in_smem = sims_smem <= 160u * 1024u;
+    // dense rows in what is left of 224 KB
+    int32_t dense_rows = 0;
+    if (ESZ == 4 && !kRepeats && sims_in_smem)
+        dense_rows = static_cast<int32_t>(std::min<size_t>(
+            kMaxDenseRows, (224u * 1024u - sims_smem) / (static_cast<size_t>(nc_row) * 4)));
+    const size_t smem =
+        sims_in_smem ? sims_smem + static_cast<size_t>(dense_rows) * nc_row * 4 : 0;
+    if (sims_in_smem)
+        cuda_check(nsp::allow_opt_in_smem(assign_kernel<ESZ, kRepeats>), "assign smem");
+    // one CTA of 32 warps per SM: as many warps as four CTAs of 8 hide
+    // the memory round trips with, and a quarter of the per-CTA term
+    // tables (trun, tcnt, ...), which then stay in L2 (8.8M SQ docs:
+    // 6.4 -> 5.5 s against four CTAs of 8 warps; two of 16: 5.7 s)
+    int per_sm = 0;
+    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, assign_kernel<ESZ, kRepeats>,
+                                                             wpb * 32, smem),
+               "assign occupancy");
+    const size_t ctas = static_cast<size_t>(nsp::device_sm_count()) * std::max(1, std::min(per_sm, 1));
+    const nsp::Arena::Mark mark = scratch.mark();
+    AssignArgs a{};
+    a.f = f;
+    a.n_lists = l.n_lists;
+    a.kept_ptr = l.kept_ptr;
+    a.kept = l.kept;
+    a.cptr = l.cptr;
+    a.cpos = l.cpos;
+    a.out_key = out_key;
+    a.max_centroid_entries = max_ce;
+    a.max_kept = std::max<int64_t>(l.max_kept, 1);
+    a.max_nc = nc_row;
+    a.dense_rows = dense_rows;
+    a.sims_in_smem = sims_in_smem ? 1 : 0;
+    a.work = scratch.take<int32_t>(1);
+    a.tcnt = scratch.take<int32_t>(ctas * dim);
+    a.tcur = scratch.take<int32_t>(ctas * dim);
+    a.trun = scratch.take<int2>(ctas * dim);
+    a.touched = scratch.take<int32_t>(ctas * max_ce);
+    a.ccl = scratch.take<uint16_t>(ctas * max_ce);
+    a.cw = scratch.take<uint8_t>(ctas * max_ce * ESZ);
+    a.is_centroid = scratch.take<uint8_t>(ctas * a.max_kept);
+    a.sims = scratch.take<uint8_t>(ctas * wpb * a.max_nc * 8);
+    cuda_check(cudaMemsetAsync(a.tcnt, 0, ctas * dim * 4, s), "memset");
+    cuda_check(cudaMemsetAsync(a.trun, 0, ctas * dim * sizeof(int2), s), "memset");
+    cuda_check(cudaMemsetAsync(a.work, 0, 4, s), "memset");
+    assign_kernel<ESZ, kRepeats><<<static_cast<unsigned>(ctas), wpb * 32, smem, s>>>(a);
+    cuda_check(cudaGetLastError(), "assign_kernel");
+    scratch.release(mark);
+}
 
 template <int ESZ>
 void build_typed(SeismicState& st, int dim, const SeismicClusterParameters& p) {
@@ -698,67 +834,22 @@ void build_typed(SeismicState& st, int dim, const SeismicClusterParameters& p) {
     for (int64_t d = 0; d < n_docs; ++d)
         max_row = std::max<int64_t>(max_row, h.indptr[d + 1] - h.indptr[d]);
     bool assigned = total_kept == 0;
+    const nsp::AssignLists lists{n_lists, d_kept_ptr, kept,     d_cptr,
+                                 d_cpos,  max_nc,     max_kept, max_row};
     if (ESZ == 1 && !assigned) {
-        const nsp::AssignLists lists{n_lists, d_kept_ptr, kept,     d_cptr,
-                                     d_cpos,  max_nc,     max_kept, max_row};
         std::vector<int64_t> df(static_cast<size_t>(n_lists));
         for (int32_t t = 0; t < n_lists; ++t) df[t] = h_post[t + 1] - h_post[t];
         assigned = nsp::assign_u8(f, lists, df, akey, s, arena);
     }
     if (!assigned) {
-        const int64_t max_ce = std::max<int64_t>(1, static_cast<int64_t>(max_nc) * max_row);
-        const int wpb = 32;
-        const size_t acc_bytes = sizeof(assign_acc_t<ESZ>);
-        const int32_t nc_row = (std::max(max_nc, 1) + 3) & ~3;
-        const size_t sims_smem = static_cast<size_t>(wpb) * nc_row * acc_bytes;
-        const bool sims_in_smem = sims_smem <= 160u * 1024u;
-        // dense rows in what is left of 224 KB
-        int32_t dense_rows = 0;
-        if (ESZ == 4 && sims_in_smem)
-            dense_rows = static_cast<int32_t>(std::min<size_t>(
-                kMaxDenseRows, (224u * 1024u - sims_smem) / (static_cast<size_t>(nc_row) * 4)));
-        const size_t smem =
-            sims_in_smem ? sims_smem + static_cast<size_t>(dense_rows) * nc_row * 4 : 0;
-        if (sims_in_smem)
-            cuda_check(nsp::allow_opt_in_smem(assign_kernel<ESZ>), "assign smem");
-        // one CTA of 32 warps per SM: as many warps as four CTAs of 8 hide
-        // the memory round trips with, and a quarter of the per-CTA term
-        // tables (trun, tcnt, ...), which then stay in L2 (8.8M SQ docs:
-        // 6.4 -> 5.5 s against four CTAs of 8 warps; two of 16: 5.7 s)
-        int per_sm = 0;
-        cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, assign_kernel<ESZ>,
-                                                                 wpb * 32, smem),
-                   "assign occupancy");
-        const size_t ctas = static_cast<size_t>(sms) * std::max(1, std::min(per_sm, 1));
-        const nsp::Arena::Mark mark = arena.mark();
-        AssignArgs a{};
-        a.f = f;
-        a.n_lists = n_lists;
-        a.kept_ptr = d_kept_ptr;
-        a.kept = kept;
-        a.cptr = d_cptr;
-        a.cpos = d_cpos;
-        a.out_key = akey;
-        a.max_centroid_entries = max_ce;
-        a.max_kept = std::max<int64_t>(max_kept, 1);
-        a.max_nc = nc_row;
-        a.dense_rows = dense_rows;
-        a.sims_in_smem = sims_in_smem ? 1 : 0;
-        a.work = arena.take<int32_t>(1);
-        a.tcnt = arena.take<int32_t>(ctas * dim);
-        a.tcur = arena.take<int32_t>(ctas * dim);
-        a.trun = arena.take<int2>(ctas * dim);
-        a.touched = arena.take<int32_t>(ctas * max_ce);
-        a.ccl = arena.take<uint16_t>(ctas * max_ce);
-        a.cw = arena.take<uint8_t>(ctas * max_ce * ESZ);
-        a.is_centroid = arena.take<uint8_t>(ctas * a.max_kept);
-        a.sims = arena.take<uint8_t>(ctas * wpb * a.max_nc * 8);
-        cuda_check(cudaMemsetAsync(a.tcnt, 0, ctas * dim * 4, s), "memset");
-        cuda_check(cudaMemsetAsync(a.trun, 0, ctas * dim * sizeof(int2), s), "memset");
-        cuda_check(cudaMemsetAsync(a.work, 0, 4, s), "memset");
-        assign_kernel<ESZ><<<static_cast<unsigned>(ctas), wpb * 32, smem, s>>>(a);
-        cuda_check(cudaGetLastError(), "assign_kernel");
-        arena.release(mark);
+        int* repeats = arena.take<int>(1);
+        cuda_check(cudaMemsetAsync(repeats, 0, sizeof(int), s), "memset");
+        repeats_kernel<<<sms * 7, kSeenWarps * 32, 0, s>>>(f, repeats);
+        cuda_check(cudaGetLastError(), "repeats_kernel");
+        if (to_host(repeats, 1, s)[0] != 0)
+            assign_general<ESZ, true>(f, lists, akey, s, arena);
+        else
+            assign_general<ESZ, false>(f, lists, akey, s, arena);
     }
 
     clock.mark("assignment");
