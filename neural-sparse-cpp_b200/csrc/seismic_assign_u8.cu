@@ -2,15 +2,15 @@
 // (cluster/kmeans_utils.cpp:40-195): every kept doc of a posting list goes to
 // the list's centroid of largest dot product, the lowest index on ties.
 //
-// Code products are integers, so a dot product may be summed in any order and
-// split: over the corpus's kHot most frequent terms it is a dense contraction
-// on the tensor cores (tcgen05.mma kind::i8, uint8 x uint8 into int32 in
-// TMEM), over the others it stays sparse. Terms are Zipf-like: two docs of
-// the SPLADE shapes share 32 terms on average, all but 0.25 of them among the
-// 1,024 most frequent, so the sparse part falls from ~32 products per (doc,
-// centroid) pair to a quarter of one, and the dense part's 1,024
-// multiply-adds per pair cost the tensor cores less than the 32 cost the
-// shared-memory pipe.
+// Code products are integers, and their sums below 2^31 for rows of up to
+// 33,025 entries, so a dot product may be summed in any order and split: over
+// the corpus's kHot most frequent terms it is a dense contraction on the
+// tensor cores (tcgen05.mma kind::i8, uint8 x uint8 into int32 in TMEM), over
+// the others it stays sparse. Terms are Zipf-like: two docs of the SPLADE
+// shapes share 32 terms on average, all but 0.25 of them among the 1,024 most
+// frequent, so the sparse part falls from ~32 products per (doc, centroid)
+// pair to a quarter of one, and the dense part's 1,024 multiply-adds per pair
+// cost the tensor cores less than the 32 cost the shared-memory pipe.
 //
 //   hot rows   every doc's codes of the hot terms as a dense row of kHot
 //              bytes in global memory (built once per build);
@@ -558,7 +558,9 @@ hot_rows_kernel(FwdView f, const uint16_t* slot_of, int hot_bytes, uint8_t* hot,
 bool assign_u8(const FwdView& f, const AssignLists& lists, const std::vector<int64_t>& df,
                uint32_t* out_key, cudaStream_t s, Arena& scratch) {
     const int dim = f.dim;
-    if (lists.max_nc > kAssignMaxCentroids || f.n_docs == 0 || dim > kMaxDim) return false;
+    if (lists.max_nc > kAssignMaxCentroids || f.n_docs == 0 || dim > kMaxDim ||
+        lists.max_row > kAssignMaxRowU8)
+        return false;
     // the hot terms: as many as the dense rows hold, by document frequency
     size_t free_b = 0, total_b = 0;
     cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");

@@ -26,10 +26,13 @@ struct AssignLists {
 // out_key[kept position] = cluster * 2 + (centroid ? 0 : 1), as assign_kernel
 // gives it. `df`: documents per term. Returns false, having written nothing,
 // where the general kernel is the one to use: a row that is not strictly
-// ascending, more than kAssignMaxCentroids centroids in a list, a vocabulary
-// past 49,152 terms, or terms so evenly spread that the frequent ones hold
-// less than half of the products.
+// ascending, or of more than kAssignMaxRowU8 entries, more than
+// kAssignMaxCentroids centroids in a list, a vocabulary past 49,152 terms, or
+// terms so evenly spread that the frequent ones hold less than half of the
+// products.
 constexpr int kAssignMaxCentroids = 1024;
+// Terms two rows can share with their sum of uint8 code products below 2^31.
+constexpr int64_t kAssignMaxRowU8 = INT32_MAX / (255 * 255);
 bool assign_u8(const FwdView& f, const AssignLists& lists, const std::vector<int64_t>& df,
                uint32_t* out_key, cudaStream_t s, Arena& scratch);
 

@@ -231,12 +231,13 @@ constexpr int kDenseShift = 20;  // counts are at most 65,536 centroids
 constexpr int kMaxDenseRows = 64;
 
 // Similarity accumulators: fp32 for fp32 values; for codes int64, or int for
-// uint8 codes of rows without repeated terms (a product per entry of the
-// doc's row).
-template <int ESZ, bool kRepeats>
+// uint8 codes of rows so short that it holds every sum: kAnyRows is set for
+// rows that repeat a term, and for uint8 rows of more than kAssignMaxRowU8
+// entries.
+template <int ESZ, bool kAnyRows>
 using assign_acc_t = typename std::conditional<
     ESZ == 4, float,
-    typename std::conditional<ESZ == 1 && !kRepeats, int, long long>::type>::type;
+    typename std::conditional<ESZ == 1 && !kAnyRows, int, long long>::type>::type;
 
 template <int ESZ>
 using assign_val_t = typename std::conditional<
@@ -281,14 +282,14 @@ __device__ __forceinline__ void apply_dense(float* sims, const float* row, float
 template <class T>
 __device__ __forceinline__ void apply_dense(T*, const float*, T, int32_t, int) {}
 
-// kRepeats: some row repeats a term. A centroid then has several entries in
+// kAnyRows: some row may repeat a term. A centroid then has several entries in
 // one term's run, which the reference adds in the centroid's order
 // (kmeans_utils.cpp:40-97): one warp indexes the centroids in order, so a run
 // lists them as they come, and entries of one centroid take turns. Other
 // indexes have distinct centroids in a run, whose products commute.
-template <int ESZ, bool kRepeats>
+template <int ESZ, bool kAnyRows>
 __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
-    using acc_t = assign_acc_t<ESZ, kRepeats>;
+    using acc_t = assign_acc_t<ESZ, kAnyRows>;
     using val_t = assign_val_t<ESZ>;
     // centroid entries of one term in flight per lane: a term's run is
     // loaded kChunks * 32 entries at a time, the next hit term's first
@@ -328,7 +329,7 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
     // of the same traffic (80,000 docs, lambda 4000, beta 400, assignment: 89
     // ms without rows, 78 with them and with four entries in flight in the
     // indexing below, 101 with the stage).
-    constexpr bool kDense = ESZ == 4 && !kRepeats;  // (a row's cell holds one entry)
+    constexpr bool kDense = ESZ == 4 && !kAnyRows;  // (a row's cell holds one entry)
     float* rows = reinterpret_cast<float*>(dyn) + static_cast<size_t>(wpb) * a.max_nc;
     const val_t* fval = static_cast<const val_t*>(a.f.val);
 
@@ -390,7 +391,7 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
             for (int32_t i = threadIdx.x; i < cells; i += blockDim.x) rows[i] = 0.0f;
             __syncthreads();
         }
-        if constexpr (kRepeats) {
+        if constexpr (kAnyRows) {
             for (int32_t c = 0; c < nc && warp == 0; ++c) {
                 const int32_t doc = a.kept[kb + cp[c]];
                 const uint2 ri = a.f.rowinfo[doc];
@@ -411,7 +412,7 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
                 }
             }
         }
-        for (int32_t c = warp; c < nc && !kRepeats; c += wpb) {
+        for (int32_t c = warp; c < nc && !kAnyRows; c += wpb) {
             const int32_t doc = a.kept[kb + cp[c]];
             const uint2 ri = a.f.rowinfo[doc];
             const int64_t rb = static_cast<int64_t>(ri.x) * nsp::kRowAlign;
@@ -506,7 +507,7 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
                     }
 #pragma unroll
                     for (int j = 0; j < kChunks; ++j) {
-                        if constexpr (kRepeats)
+                        if constexpr (kAnyRows)
                             add_products_in_turn(sims, cc[j], cdv, cwv[j], lane);
                         else if (cc[j] >= 0)
                             add_product(sims, cc[j], cdv, cwv[j]);
@@ -523,7 +524,7 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
                         }
 #pragma unroll
                         for (int j = 0; j < kChunks; ++j) {
-                            if constexpr (kRepeats)
+                            if constexpr (kAnyRows)
                                 add_products_in_turn(sims, cc[j], cdv, cwv[j], lane);
                             else if (cc[j] >= 0)
                                 add_product(sims, cc[j], cdv, cwv[j]);
@@ -673,31 +674,31 @@ struct PhaseClock {
 };
 
 // Assignment by assign_kernel: any values, any rows.
-template <int ESZ, bool kRepeats>
+template <int ESZ, bool kAnyRows>
 void assign_general(const nsp::FwdView& f, const nsp::AssignLists& l, uint32_t* out_key,
                     cudaStream_t s, nsp::Arena& scratch) {
     const int dim = f.dim;
     const int64_t max_ce = std::max<int64_t>(1, static_cast<int64_t>(l.max_nc) * l.max_row);
     const int wpb = 32;
-    const size_t acc_bytes = sizeof(assign_acc_t<ESZ, kRepeats>);
+    const size_t acc_bytes = sizeof(assign_acc_t<ESZ, kAnyRows>);
     const int32_t nc_row = (std::max(l.max_nc, 1) + 3) & ~3;
     const size_t sims_smem = static_cast<size_t>(wpb) * nc_row * acc_bytes;
     const bool sims_in_smem = sims_smem <= 160u * 1024u;
     // dense rows in what is left of 224 KB
     int32_t dense_rows = 0;
-    if (ESZ == 4 && !kRepeats && sims_in_smem)
+    if (ESZ == 4 && !kAnyRows && sims_in_smem)
         dense_rows = static_cast<int32_t>(std::min<size_t>(
             kMaxDenseRows, (224u * 1024u - sims_smem) / (static_cast<size_t>(nc_row) * 4)));
     const size_t smem =
         sims_in_smem ? sims_smem + static_cast<size_t>(dense_rows) * nc_row * 4 : 0;
     if (sims_in_smem)
-        cuda_check(nsp::allow_opt_in_smem(assign_kernel<ESZ, kRepeats>), "assign smem");
+        cuda_check(nsp::allow_opt_in_smem(assign_kernel<ESZ, kAnyRows>), "assign smem");
     // one CTA of 32 warps per SM: as many warps as four CTAs of 8 hide
     // the memory round trips with, and a quarter of the per-CTA term
     // tables (trun, tcnt, ...), which then stay in L2 (8.8M SQ docs:
     // 6.4 -> 5.5 s against four CTAs of 8 warps; two of 16: 5.7 s)
     int per_sm = 0;
-    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, assign_kernel<ESZ, kRepeats>,
+    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, assign_kernel<ESZ, kAnyRows>,
                                                              wpb * 32, smem),
                "assign occupancy");
     const size_t ctas = static_cast<size_t>(nsp::device_sm_count()) * std::max(1, std::min(per_sm, 1));
@@ -727,7 +728,7 @@ void assign_general(const nsp::FwdView& f, const nsp::AssignLists& l, uint32_t* 
     cuda_check(cudaMemsetAsync(a.tcnt, 0, ctas * dim * 4, s), "memset");
     cuda_check(cudaMemsetAsync(a.trun, 0, ctas * dim * sizeof(int2), s), "memset");
     cuda_check(cudaMemsetAsync(a.work, 0, 4, s), "memset");
-    assign_kernel<ESZ, kRepeats><<<static_cast<unsigned>(ctas), wpb * 32, smem, s>>>(a);
+    assign_kernel<ESZ, kAnyRows><<<static_cast<unsigned>(ctas), wpb * 32, smem, s>>>(a);
     cuda_check(cudaGetLastError(), "assign_kernel");
     scratch.release(mark);
 }
@@ -846,7 +847,7 @@ void build_typed(SeismicState& st, int dim, const SeismicClusterParameters& p) {
         cuda_check(cudaMemsetAsync(repeats, 0, sizeof(int), s), "memset");
         repeats_kernel<<<sms * 7, kSeenWarps * 32, 0, s>>>(f, repeats);
         cuda_check(cudaGetLastError(), "repeats_kernel");
-        if (to_host(repeats, 1, s)[0] != 0)
+        if (to_host(repeats, 1, s)[0] != 0 || (ESZ == 1 && max_row > nsp::kAssignMaxRowU8))
             assign_general<ESZ, true>(f, lists, akey, s, arena);
         else
             assign_general<ESZ, false>(f, lists, akey, s, arena);
