@@ -524,13 +524,14 @@ __global__ void __launch_bounds__(1024, 1) seismic_cluster_kernel(SeismicLaunch 
                         }
                         ++lists;
                         const size_t pairs = static_cast<size_t>(nb) * sizeof(ranking::Blk);
+                        const size_t sort_room = L.sq - L.cdoc;
                         ranking::Blk* items = reinterpret_cast<ranking::Blk*>(
-                            pairs <= room ? reinterpret_cast<unsigned long long*>(cdoc) : keys_g);
+                            pairs <= sort_room ? reinterpret_cast<unsigned long long*>(cdoc) : keys_g);
                         if (items == nullptr) {  // the host sizes sortkeys; never taken
                             if (tid == 0) atomicExch(a.err, 2);
                             break;
                         }
-                        uint16_t* stops = pairs + static_cast<size_t>(nb) * 2 <= room
+                        uint16_t* stops = pairs + static_cast<size_t>(nb) * 2 <= sort_room
                                               ? reinterpret_cast<uint16_t*>(smem + L.cdoc + pairs)
                                               : order;
                         sort_blocks(bscore + static_cast<size_t>(s) * maxb, nb, items, stops, order,

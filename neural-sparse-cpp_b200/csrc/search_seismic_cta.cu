@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(1024, 1) seismic_cta_kernel(SeismicLaunch a) {
                 int nbv = nb;
                 if (first) {
                     // in the batch arrays' place where they are large enough
-                    const size_t room = L.wsum - L.cdoc;
+                    const size_t room = L.sq - L.cdoc;
                     const size_t pairs = static_cast<size_t>(nb) * sizeof(ranking::Blk);
                     ranking::Blk* items = reinterpret_cast<ranking::Blk*>(
                         pairs <= room ? reinterpret_cast<unsigned long long*>(cdoc) : keys_g);

@@ -26,6 +26,7 @@ using detail_search::ValT;
 
 constexpr int kSegCap = 128;    // block segments per batch, one CTA per query
 constexpr int kSortQueue = 64;  // ranges sorted side by side (two per warp at most)
+constexpr size_t kSortQueueBytes = 2 * kSortQueue * 4 + 16;  // both queues and their sizes
 constexpr int kSegCapMax = 1024;  // the most any launch asks for (a cluster per query)
 
 // A run of consecutive docs of one block inside a batch.
@@ -63,12 +64,14 @@ struct Ctl {
 __host__ __device__ inline size_t a16(size_t x) { return (x + 15) & ~size_t(15); }
 
 struct CtaLayout {
-    size_t tbl, qv, qterm, qraw, cuts, hs, hid, cdoc, coff, clen, csc, segs, cseg, wsum, cur, uq,
-        sq, total;
+    size_t tbl, qv, qterm, qraw, cuts, hs, hid, cdoc, coff, clen, csc, segs, cseg, sq, wsum, cur,
+        uq, total;
 };
 
 // Shared-memory layout of one CTA. The four candidate arrays are contiguous
-// (16 * batch bytes) and double as the sort-key buffer of the first list.
+// (16 * batch bytes) and double as the sort-key buffer of the first list; the
+// sort's queue takes the end of the segments' place, so that the largest k and
+// the longest query that fit depend on the arrays above alone.
 __host__ __device__ inline CtaLayout cta_layout(int vsize, int tsize, int dim, int qcap, int k,
                                                 int batch, int seg_cap) {
     CtaLayout L;
@@ -86,10 +89,10 @@ __host__ __device__ inline CtaLayout cta_layout(int vsize, int tsize, int dim, i
     L.csc = o;   o += static_cast<size_t>(batch) * 4;
     L.segs = o;  o += static_cast<size_t>(seg_cap) * sizeof(Seg);
     L.cseg = o;  o += a16(static_cast<size_t>(batch) * 2);
+    L.sq = o - kSortQueueBytes;  // (kSegCap segments alone are more)
     L.wsum = o;  o += 32 * 4;
     L.cur = o;   o += 64;  // warp 0's Cursor
     L.uq = o;    o += 2 * 32 * 4;  // counting pass: warp 0's per-lane unique docs, row bytes
-    L.sq = o;    o += 2 * kSortQueue * 4 + 16;  // ranges of the first list's sort
     L.total = o;
     return L;
 }
