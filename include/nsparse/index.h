@@ -24,7 +24,8 @@ struct EngineOptions {
     // loading doc rows straight from HBM, 1 the same with rows staged in
     // shared memory by bulk copy (stage_bytes per buffer, 0 = default), 2-5
     // one CTA per query with 1, 2, 4 or 8 lanes per scored doc, in batches of
-    // batch_docs candidate docs (0 = default). Results are identical.
+    // batch_docs candidate docs (0 = default); a cluster of CTAs per query
+    // takes eight lanes with each of 2-5. Results are identical.
     int variant = -1;
     int stage_bytes = 0;
     int batch_docs = 0;

@@ -150,9 +150,10 @@ nsp_status_t nsp_search_params_set_engine(nsp_search_params_t* params, int plain
                                           int warps_per_block);
 /* Extension: SEISMIC kernel variant (-1 engine's choice, 0 one warp per query
  * with direct row loads, 1 the same with rows staged in shared memory by bulk
- * copy, 2-5 one CTA per query with 1, 2, 4 or 8 lanes per scored doc) and its
- * tuning value: variant 1's buffer size in bytes, variants 2-5's candidate
- * docs per batch (0 = default). Results do not depend on either. */
+ * copy, 2-5 one CTA per query with 1, 2, 4 or 8 lanes per scored doc -- a
+ * cluster of CTAs per query takes eight with each of them) and its tuning
+ * value: variant 1's buffer size in bytes, variants 2-5's candidate docs per
+ * batch (0 = default). Results do not depend on either. */
 nsp_status_t nsp_search_params_set_kernel(nsp_search_params_t* params, int variant,
                                           int tuning);
 /* Extension: CTAs per query of SEISMIC variants 2-5 (0 engine's choice, 1 one
@@ -238,11 +239,11 @@ nsp_status_t nsp_index_search_device_noalloc(nsp_index_t* index, int32_t n,
 /* Kernel autotuner. Times each one-CTA-per-query launch shape of the SEISMIC
  * search (lanes per doc, candidate docs per batch, warps per CTA) on the n
  * sample queries with the given parameters, then the CTAs per query (1, 2, 4,
- * 8) of one-query launches on up to 16 of them searched alone, and keeps the
- * fastest for this index: later searches whose parameters leave the kernel to
- * the engine (variant -1) use it. Results do not depend on the choice. Writes
- * the choice to the out pointers (any may be NULL). Extension with no
- * counterpart in the reference. */
+ * 8 and the engine's own choice, reported as at most 8) of one-query launches
+ * on up to 16 of them searched alone, and keeps the fastest for this index:
+ * later searches whose parameters leave the kernel to the engine (variant -1)
+ * use it. Results do not depend on the choice. Writes the choice to the out
+ * pointers (any may be NULL). Extension with no counterpart in the reference. */
 nsp_status_t nsp_index_autotune(nsp_index_t* index, int32_t n, const int32_t* indptr,
                                 const uint16_t* indices, const float* values, int k,
                                 const nsp_search_params_t* params, int* variant, int* batch_docs,

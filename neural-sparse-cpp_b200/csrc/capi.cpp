@@ -2,6 +2,7 @@
 // here and mapped to status codes; the message is kept per thread.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstring>
 #include <memory>
 #include <new>
@@ -372,7 +373,8 @@ nsp_status_t nsp_index_autotune(nsp_index_t* index, int32_t n, const int32_t* in
         if (batch_docs != nullptr) *batch_docs = c.batch_docs;
         if (warps_per_block != nullptr) *warps_per_block = c.warps_per_block;
         if (kernel_ms != nullptr) *kernel_ms = c.kernel_ms;
-        if (ctas_per_query != nullptr) *ctas_per_query = c.split;
+        // (16, the engine's own, is no value that a caller can ask for)
+        if (ctas_per_query != nullptr) *ctas_per_query = std::min(c.split, 8);
     });
 }
 

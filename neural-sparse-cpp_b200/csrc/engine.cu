@@ -658,9 +658,11 @@ SeismicPlan plan_seismic_cta(int kind, int dim, int qcap, int k, int n_queries,
         while (batch > 32 && seismic_cta_smem(kind, dim, qcap, k, batch, seg_cap) > limit)
             batch >>= 1;
         p.smem_cta = seismic_cta_smem(kind, dim, qcap, k, batch, seg_cap);
-        // a cluster's larger segment table (and its kernel's static shared
-        // memory, below 2 KB) must not refuse a query that one CTA can run
         if (cl == 1 || p.smem_cta + 2048 <= limit) break;
+        // a cluster's larger segment table must not refuse a query that one
+        // CTA can run, unless the caller asked for the cluster; its kernel's
+        // static shared memory, below 2 KB, must not refuse any
+        if (args.cluster > 0 && !args.cluster_may_shrink && p.smem_cta > limit) break;
         cl = 1;
     }
     if (p.smem_cta > limit)

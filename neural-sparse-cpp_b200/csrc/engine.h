@@ -314,7 +314,7 @@ struct KernelChoice {
     int batch_docs = 0;
     int warps_per_block = 0;
     float kernel_ms = 0.0f;  // on the tuning sample
-    int split = 0;           // CTAs per query of one-query launches (0: the engine's rule)
+    int split = 0;           // CTAs per query of one-query launches, up to 16 (0: the engine's rule)
 };
 
 // CTAs per query the engine gives a launch of `n_queries` queries: the most
@@ -338,7 +338,8 @@ struct SeismicSearchArgs {
                               // 2-5 one CTA per query with 1, 2, 4, 8 lanes per doc
     int stage_bytes = 0;      // staged: bytes per stage buffer (0 = default)
     int batch_docs = 0;       // variants 2-5: candidate docs per batch (0 = default)
-    int cluster = 0;          // variants 2-5: CTAs per query (0 = engine's choice up to 16, 1, 2, 4, 8)
+    int cluster = 0;          // variants 2-5: CTAs per query (0 = the engine's rule, up to 16)
+    bool cluster_may_shrink = false;  // `cluster` is the engine's choice: fewer where it does not fit
     // variants 2-5: one device doc bitmap per query (a null entry admits every
     // doc), in device memory; replaces the launch-wide selector
     const uint64_t* const* d_sel_q = nullptr;

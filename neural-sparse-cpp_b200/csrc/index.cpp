@@ -388,11 +388,11 @@ void apply_tuned(const SeismicState& st, nsp::SeismicSearchArgs& a, int64_t n_qu
     a.variant = st.tuned.variant;
     if (a.cluster == 0 && st.tuned.split > 0) {
         // the split measured fastest for a lone query, where the engine's
-        // rule would give a launch this small a cluster at all (the largest
-        // split measured leaves the rule its own choice)
+        // rule would give a launch this small a cluster at all
         const int rule = nsp::auto_cluster(
             a.plain ? 1 : static_cast<int>(std::min<int64_t>(n_queries, 1 << 30)));
-        a.cluster = st.tuned.split < 8 ? std::min(rule, st.tuned.split) : rule;
+        a.cluster = std::min(rule, st.tuned.split);
+        a.cluster_may_shrink = true;
     }
     if (a.plain || n_queries <= 2 * static_cast<int64_t>(nsp::device_sm_count())) return;
     if (a.batch_docs == 0) a.batch_docs = st.tuned.batch_docs;
@@ -767,15 +767,20 @@ nsp::KernelChoice seismic_autotune(Index* index, idx_t n, const idx_t* indptr,
         }
     }
     // CTAs per query for one-query launches (the latency of a lone query):
-    // the fastest of 1, 2, 4, 8 over up to 16 of the sample's queries, each
-    // searched alone with the chosen lanes per doc
+    // the fastest of 1, 2, 4, 8 and the rule's own choice over up to 16 of the
+    // sample's queries, each searched alone (one CTA with the chosen lanes per
+    // doc; a cluster has eight always)
     const int n1 = std::min<int>(n, 16);
     float best_ms = 0.0f;
-    for (int split : {1, 2, 4, 8}) {
+    int timed = 0;
+    for (int split : {1, 2, 4, 8, nsp::auto_cluster(1)}) {
+        if (split <= timed) continue;
+        timed = split;
         nsp::SeismicSearchArgs t = a;
         t.variant = best.variant;
         t.plain = true;
         t.cluster = split;
+        t.cluster_may_shrink = true;
         float total = 0.0f;
         for (int rep = 0; rep < 2; ++rep) {  // the first pass warms caches
             total = 0.0f;

@@ -179,7 +179,7 @@ extern "C" nsp_status_t nsp_index_search_device_noalloc(
             return static_cast<long long>((avail - nd.fixed - slack) / nd.per_cta);
         };
         long long room = fits(need);
-        const bool engines_choice = a.cluster <= 0;
+        const bool engines_choice = a.cluster <= 0 || a.cluster_may_shrink;
         while (room < need.cluster && need.cluster > 1 && engines_choice) {
             // the engine's cluster does not fit: smaller ones (past 8 CTAs),
             // then one CTA per query

@@ -369,10 +369,12 @@ void Server::worker() {
             resolve_seismic(index_, &params, k, a);
             // CTAs per query by the queries on the GPU at once, this batch's
             // and the other workers': a cluster per query only while the SMs
-            // would otherwise idle (capped by the autotuner's split)
+            // would otherwise idle (capped by the autotuner's split, and at 8:
+            // a cluster of 16 takes most of a GPC from the other workers)
             a.cluster = std::min(
                 nsp::auto_cluster(static_cast<int>(std::min<int64_t>(others + n, 1 << 30))),
-                st_->tuned.split > 0 ? st_->tuned.split : 8);
+                st_->tuned.split > 0 ? std::min(st_->tuned.split, 8) : 8);
+            a.cluster_may_shrink = true;
             apply_tuned(*st_, a, static_cast<int64_t>(batch.size()));
             if (a.variant >= 0 && a.variant < 2) a.variant = -1;  // needs one CTA per query
             const bool any =
