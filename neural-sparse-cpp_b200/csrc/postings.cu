@@ -25,13 +25,6 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 
-// A term's postings are applied with a shared-memory read-modify-write each
-// (about 10 L1 wavefronts per 32 postings, random banks), its dense row with
-// 12 wavefronts per 128 docs, fewer in a run of dense terms: dense is cheaper
-// from about 0.3 of the docs on. 256 rows bound the memory at 1 KB per doc.
-constexpr double kDenseShare = 0.3;
-constexpr size_t kMaxDense = 256;
-
 // off[d] = row d's length; *unsorted = 1 if some row's terms are not
 // strictly ascending. One warp per row.
 __global__ void row_lens_kernel(FwdView f, int64_t* off, int* unsorted) {
@@ -179,10 +172,12 @@ void PostingsDevice::build(const ForwardDevice& fwd, int chunk_docs) {
     doc_.resize(static_cast<size_t>(std::max<int64_t>(nnz, 1)));
     val_.resize(static_cast<size_t>(std::max<int64_t>(nnz, 1)));
     if (nnz > 0) {
-        uint16_t* k_in = scratch.take<uint16_t>(static_cast<size_t>(nnz));
-        uint16_t* k_out = scratch.take<uint16_t>(static_cast<size_t>(nnz));
-        auto* v_in = scratch.take<unsigned long long>(static_cast<size_t>(nnz));
-        auto* v_out = scratch.take<unsigned long long>(static_cast<size_t>(nnz));
+        // (given back before the arrays below are allocated)
+        Arena sort(s);
+        uint16_t* k_in = sort.take<uint16_t>(static_cast<size_t>(nnz));
+        uint16_t* k_out = sort.take<uint16_t>(static_cast<size_t>(nnz));
+        auto* v_in = sort.take<unsigned long long>(static_cast<size_t>(nnz));
+        auto* v_out = sort.take<unsigned long long>(static_cast<size_t>(nnz));
         compact_kernel<<<grid_for(static_cast<int64_t>(n) * 32, 256), 256, 0, s>>>(
             f, off, k_in, v_in);
         cuda_check(cudaGetLastError(), "compact_kernel");
@@ -191,7 +186,7 @@ void PostingsDevice::build(const ForwardDevice& fwd, int chunk_docs) {
                                                    v_in, v_out, static_cast<int>(nnz),
                                                    0, 16, s),
                    "radix sort size");
-        auto* tmp = scratch.take<unsigned char>(tmp_bytes);
+        auto* tmp = sort.take<unsigned char>(tmp_bytes);
         cuda_check(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, k_in, k_out,
                                                    v_in, v_out, static_cast<int>(nnz),
                                                    0, 16, s),
@@ -210,28 +205,30 @@ void PostingsDevice::build(const ForwardDevice& fwd, int chunk_docs) {
     chunk_at_kernel<<<grid_for(static_cast<int64_t>(dim) * (n_chunks_ + 1), 256), 256, 0, s>>>(
         tstart, doc_.data(), dim, n_chunks_, chunk_docs, chunk_at_.data());
     cuda_check(cudaGetLastError(), "chunk_at_kernel");
-    // the frequent terms, most frequent first
+    // dense rows of the frequent terms, as far as there is memory for them
     std::vector<int32_t> h_start(static_cast<size_t>(dim) + 1);
     cuda_check(cudaMemcpyAsync(h_start.data(), tstart, h_start.size() * sizeof(int32_t),
                                cudaMemcpyDeviceToHost, s), "D2H");
     cuda_check(cudaStreamSynchronize(s), "sync");
-    std::vector<int32_t> frequent;
-    for (int32_t t = 0; t < dim; ++t)
-        if (h_start[t + 1] - h_start[t] >= kDenseShare * n && h_start[t + 1] > h_start[t])
-            frequent.push_back(t);
-    std::sort(frequent.begin(), frequent.end(), [&](int32_t x, int32_t y) {
-        const int32_t dx = h_start[x + 1] - h_start[x], dy = h_start[y + 1] - h_start[y];
-        return dx != dy ? dx > dy : x < y;
-    });
-    if (frequent.size() > kMaxDense) frequent.resize(kMaxDense);
+    const size_t row_cells = static_cast<size_t>(n_chunks_) * chunk_docs;
+    size_t free_b = 0, total_b = 0;
+    cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
+    std::vector<int32_t> frequent = dense_terms(h_start, n, row_cells * sizeof(float), free_b);
+    frequent.resize(allocate_dense_rows(frequent.size(), [&](size_t rows) {
+        try {
+            dense_.resize(rows * row_cells);
+        } catch (...) {
+            (void)cudaGetLastError();  // the failed allocation's
+            throw;
+        }
+    }));
     n_dense_ = static_cast<int32_t>(frequent.size());
     std::vector<int16_t> of(static_cast<size_t>(std::max(dim, 1)), -1);
     for (int32_t j = 0; j < n_dense_; ++j) of[frequent[j]] = static_cast<int16_t>(j);
     dense_of_.upload(of.data(), of.size(), s);
     if (n_dense_ > 0) {
-        const size_t cells = static_cast<size_t>(n_chunks_) * n_dense_ * chunk_docs;
-        dense_.resize(cells);
-        cuda_check(cudaMemsetAsync(dense_.data(), 0, cells * sizeof(float), s), "memset");
+        cuda_check(cudaMemsetAsync(dense_.data(), 0, n_dense_ * row_cells * sizeof(float), s),
+                   "memset");
         const int32_t* terms = scratch.put(frequent.data(), frequent.size());
         dense_rows_kernel<<<dim3(static_cast<unsigned>(grid_for(n, 256 * 8)),
                                  static_cast<unsigned>(n_dense_)), 256, 0, s>>>(
