@@ -14,6 +14,7 @@
 #include <string>
 #include <utility>
 
+#include "postings_plan.h"
 #include "scan.h"
 
 namespace nsp {
@@ -1093,12 +1094,24 @@ void exact_search(const ForwardDevice& fwd, const PostingsDevice* post, const Qu
     if (taat) {
         // term at a time: candidates per (query, doc chunk), no per-lane lists
         a.post = post->view();
-        // (non-finite query values can give NaN scores, whose order depends
-        // on the parts: they keep whole chunks)
+        // Dense rows need finite query values (a doc without the term adds a
+        // zero product). NaN scores, of non-finite or very large values in
+        // queries or docs, have no rank, so their order depends on the parts:
+        // chunks stay whole wherever there can be one, whatever the batch.
         bool finite = true;
-        for (int64_t i = q.ip[0]; i < q.ip[q.n]; ++i) finite &= std::isfinite(q.vv[i]);
+        double query_abs = 0.0;
+        for (int32_t i = 0; i < q.n; ++i) {
+            double sum = 0.0;
+            for (int64_t e = q.ip[i]; e < q.ip[i + 1]; ++e) {
+                sum += std::fabs(static_cast<double>(q.vv[e]));
+                finite &= std::isfinite(q.vv[e]);
+            }
+            query_abs = std::max(query_abs, sum);
+        }
         a.dense = finite && a.post.n_dense > 0;
-        a.splits = finite ? exact_taat_splits(q.n, a.post.n_chunks, a.post.chunk_docs, sms) : 1;
+        a.ranked = finite && finite_scores(post->max_abs(), query_abs);
+        a.splits =
+            a.ranked ? exact_taat_splits(q.n, a.post.n_chunks, a.post.chunk_docs, sms) : 1;
         const size_t cands = static_cast<size_t>(q.n) * a.post.n_chunks * a.splits * k;
         a.cand_d = static_cast<float*>(ws.dev(Workspace::kCandD, cands * sizeof(float)));
         a.cand_l = static_cast<int32_t*>(ws.dev(Workspace::kCandL, cands * sizeof(int32_t)));

@@ -209,10 +209,12 @@ public:
     uint64_t generation() const { return generation_; }  // of the forward index it mirrors
     PostingsView view() const;
     size_t device_bytes() const;
+    float max_abs() const { return max_abs_; }  // largest magnitude stored (NaN if any is)
 
 private:
     uint64_t generation_ = 0;
     bool usable_ = false;
+    float max_abs_ = 0.0f;
     int32_t n_chunks_ = 0;
     int32_t chunk_docs_ = 0;
     int32_t n_dense_ = 0;

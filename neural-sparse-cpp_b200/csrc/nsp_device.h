@@ -179,6 +179,7 @@ struct ExactLaunch {
     PostingsView post;          // term-at-a-time path (launch_exact_taat)
     int splits;                 // CTAs per doc chunk on that path (a divisor of its docs)
     bool dense;                 // frequent terms from their dense rows (finite weights)
+    bool ranked;                // every score is known to be finite
     QueryView q;
     int k;
     int mode;                   // 0 brutal (all docs), 1 inverted (score > 0)

@@ -76,14 +76,20 @@ __global__ void term_start_kernel(const uint16_t* keys, int64_t nnz, int dim, in
     tstart[t] = static_cast<int32_t>(lo);
 }
 
-__global__ void unpack_kernel(const unsigned long long* v, int64_t nnz, int32_t* doc, float* val) {
+// *max_abs = the bits of the largest magnitude, NaN above all (0 on entry).
+__global__ void unpack_kernel(const unsigned long long* v, int64_t nnz, int32_t* doc, float* val,
+                              unsigned* max_abs) {
+    unsigned mine = 0u;
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
     for (int64_t j = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; j < nnz;
          j += stride) {
         const unsigned long long x = v[j];
         doc[j] = static_cast<int32_t>(static_cast<uint32_t>(x));
         val[j] = __uint_as_float(static_cast<uint32_t>(x >> 32));
+        mine = max(mine, static_cast<uint32_t>(x >> 32) & 0x7fffffffu);
     }
+    mine = __reduce_max_sync(kFull, mine);
+    if ((threadIdx.x & 31) == 0 && mine > 0u) atomicMax(max_abs, mine);
 }
 
 // chunk_at[t * (nc + 1) + c] = first posting of term t with doc >= c * C.
@@ -169,6 +175,8 @@ void PostingsDevice::build(const ForwardDevice& fwd, int chunk_docs) {
     n_chunks_ = (n + chunk_docs - 1) / chunk_docs;
     const int dim = f.dim;
     int32_t* tstart = scratch.take<int32_t>(static_cast<size_t>(dim) + 1);
+    unsigned* max_abs = scratch.take<unsigned>(1);
+    cuda_check(cudaMemsetAsync(max_abs, 0, sizeof(unsigned), s), "memset");
     doc_.resize(static_cast<size_t>(std::max<int64_t>(nnz, 1)));
     val_.resize(static_cast<size_t>(std::max<int64_t>(nnz, 1)));
     if (nnz > 0) {
@@ -195,7 +203,7 @@ void PostingsDevice::build(const ForwardDevice& fwd, int chunk_docs) {
                                                                 tstart);
         cuda_check(cudaGetLastError(), "term_start_kernel");
         unpack_kernel<<<grid_for(nnz, 256), 256, 0, s>>>(v_out, nnz, doc_.data(),
-                                                         val_.data());
+                                                         val_.data(), max_abs);
         cuda_check(cudaGetLastError(), "unpack_kernel");
     } else {
         cuda_check(cudaMemsetAsync(tstart, 0, (static_cast<size_t>(dim) + 1) * 4, s),
@@ -209,6 +217,8 @@ void PostingsDevice::build(const ForwardDevice& fwd, int chunk_docs) {
     std::vector<int32_t> h_start(static_cast<size_t>(dim) + 1);
     cuda_check(cudaMemcpyAsync(h_start.data(), tstart, h_start.size() * sizeof(int32_t),
                                cudaMemcpyDeviceToHost, s), "D2H");
+    cuda_check(cudaMemcpyAsync(&max_abs_, max_abs, sizeof(max_abs_), cudaMemcpyDeviceToHost, s),
+               "D2H");
     cuda_check(cudaStreamSynchronize(s), "sync");
     const size_t row_cells = static_cast<size_t>(n_chunks_) * chunk_docs;
     size_t free_b = 0, total_b = 0;

@@ -34,6 +34,14 @@ NSP_POSTINGS_HD inline void each_posting(int32_t lo, int32_t hi, int64_t first, 
     for (int64_t p = lo + first; p < hi; p += step) visit(static_cast<int32_t>(p));
 }
 
+// Whether no score can leave the finite numbers: a bound on every partial sum
+// of products from the largest magnitude stored and the largest sum of a
+// query's magnitudes (65,536 roundings add less than half a percent). Not so
+// where either is infinite or NaN.
+inline bool finite_scores(float max_abs, double query_abs) {
+    return static_cast<double>(max_abs) * query_abs < 3.0e38;
+}
+
 // Which terms also get a dense row. A term's postings are applied with a
 // shared-memory read-modify-write each (about 10 L1 wavefronts per 32
 // postings, random banks), its dense row with 12 wavefronts per 128 docs,

@@ -763,10 +763,12 @@ __global__ void __launch_bounds__(kTThreads) exact_taat_kernel(ExactLaunch a) {
 
 // The final top k of a query's candidates (each tile's sorted, the tiles in
 // doc order, so equal scores come lowest id first), k <= kTaatMaxK, by a CTA
-// per query; NaN scores, which have no rank, are left to the one-warp merge.
+// per query. Unless all scores are known to be finite (`ranked`), a tile with
+// NaN scores, which have no rank, may have left NaN among its candidates or
+// the others unsorted: the one-warp merge takes those as they stand.
 __global__ void __launch_bounds__(kTThreads)
-exact_select_kernel(const float* cand_d, const int32_t* cand_l, int tiles, int k, float* out_d,
-                    int32_t* out_l) {
+exact_select_kernel(const float* cand_d, const int32_t* cand_l, int tiles, int k, bool ranked,
+                    float* out_d, int32_t* out_l) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint32_t bins[kBins];
     __shared__ unsigned long long words[kTaatMaxK];
@@ -776,9 +778,10 @@ exact_select_kernel(const float* cand_d, const int32_t* cand_l, int tiles, int k
     const int n = tiles * k;
     const float* cd = cand_d + static_cast<size_t>(q) * n;
     const int32_t* cl = cand_l + static_cast<size_t>(q) * n;
-    bool nan = false;
-    for (int i = threadIdx.x; i < n; i += kTThreads) nan |= cd[i] != cd[i];
-    if (__syncthreads_or(nan)) {
+    bool merge = false;
+    for (int i = threadIdx.x; i < n && !ranked; i += kTThreads)
+        merge |= cd[i] != cd[i] || ((i + 1) % k != 0 && cd[i] < cd[i + 1]);
+    if (__syncthreads_or(merge)) {
         if (threadIdx.x < 32)
             merge_candidates(cd, cl, tiles, k, reinterpret_cast<int*>(smem), threadIdx.x,
                              out_d + static_cast<size_t>(q) * k, out_l + static_cast<size_t>(q) * k);
@@ -800,7 +803,7 @@ cudaError_t merge_launch(const ExactLaunch& a, int tiles, cudaStream_t s) {
     if (a.k <= kTaatMaxK && static_cast<long long>(tiles) * a.k <= INT_MAX &&
         heads + 12 * 1024 <= 48 * 1024)
         exact_select_kernel<<<a.q.n, kTThreads, heads, s>>>(a.cand_d, a.cand_l, tiles, a.k,
-                                                            a.out_d, a.out_l);
+                                                            a.ranked, a.out_d, a.out_l);
     else
         exact_merge_kernel<<<a.q.n, 32, heads, s>>>(a.cand_d, a.cand_l, tiles, a.k, a.out_d,
                                                     a.out_l);
