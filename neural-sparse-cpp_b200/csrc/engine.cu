@@ -14,6 +14,7 @@
 #include <string>
 #include <utility>
 
+#include "arena_plan.h"
 #include "postings_plan.h"
 #include "scan.h"
 
@@ -73,14 +74,18 @@ void* Arena::bytes(size_t n) {
         used_ = 0;
     }
     if (cur_ == chunks_.size()) {
-        // each chunk twice the one before, 64 MB to 1 GB, so a small build
-        // holds little and a large one needs few
-        size_t cap = size_t{64} << 20;
-        if (!chunks_.empty())
-            cap = std::min(std::max(cap, 2 * chunks_.back().cap), size_t{1} << 30);
-        cap = std::max(cap, n);
-        void* p = nullptr;
-        cuda_check(cudaMalloc(&p, cap), "arena cudaMalloc");
+        size_t cap = arena_chunk(chunks_.empty() ? 0 : chunks_.back().cap, n);
+        cudaError_t e = cudaSuccess;
+        void* p = arena_allocate(cap, n, [&](size_t bytes) {
+            void* q = nullptr;
+            e = cudaMalloc(&q, bytes);
+            if (e != cudaSuccess) {
+                q = nullptr;
+                (void)cudaGetLastError();
+            }
+            return q;
+        });
+        cuda_check(e, "arena cudaMalloc");
         chunks_.push_back({static_cast<char*>(p), cap});
         used_ = 0;
     }
