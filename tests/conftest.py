@@ -8,6 +8,8 @@ vectors and the reference, the C ABI's host-side behaviour, and index files.
 import os
 import sys
 
+import pytest
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 for p in (os.path.join(ROOT, "neural-sparse-cpp_b200", "python"), os.path.join(ROOT, "oracle"),
           os.path.join(ROOT, "tests")):
@@ -17,3 +19,17 @@ for p in (os.path.join(ROOT, "neural-sparse-cpp_b200", "python"), os.path.join(R
 
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (B200)")
+
+
+@pytest.fixture(scope="session", autouse=True)
+def reference_or_skip():
+    """Tests that open the compiled reference are skipped where it is not built
+    (its sources are not part of this repository)."""
+    import oracle
+    if oracle.ref_available():
+        yield
+        return
+    with pytest.MonkeyPatch.context() as m:
+        m.setattr(oracle, "ref_lib",
+                  lambda variant="generic": pytest.skip("reference library not built"))
+        yield
