@@ -1103,18 +1103,19 @@ void exact_search(const ForwardDevice& fwd, const PostingsDevice* post, const Qu
         // zero product). NaN scores, of non-finite or very large values in
         // queries or docs, have no rank, so their order depends on the parts:
         // chunks stay whole wherever there can be one, whatever the batch.
-        bool finite = true;
-        double query_abs = 0.0;
-        for (int32_t i = 0; i < q.n; ++i) {
-            double sum = 0.0;
-            for (int64_t e = q.ip[i]; e < q.ip[i + 1]; ++e) {
-                sum += std::fabs(static_cast<double>(q.vv[e]));
-                finite &= std::isfinite(q.vv[e]);
-            }
-            query_abs = std::max(query_abs, sum);
+        // (Magnitudes compare as their bits, in a loop that vectorizes: a sum
+        // per query was 10 us of a call of 1,000.)
+        int32_t largest = 0;
+        for (int64_t e = q.ip[0]; e < q.ip[q.n]; ++e) {
+            int32_t bits;
+            std::memcpy(&bits, q.vv + e, sizeof(bits));
+            largest = std::max(largest, bits & 0x7fffffff);
         }
-        a.dense = finite && a.post.n_dense > 0;
-        a.ranked = finite && finite_scores(post->max_abs(), query_abs);
+        float query_max;
+        std::memcpy(&query_max, &largest, sizeof(query_max));
+        a.dense = std::isfinite(query_max) && a.post.n_dense > 0;
+        a.ranked = finite_scores(post->max_abs(),
+                                 static_cast<double>(query_max) * std::max(q.max_nnz, 1));
         a.splits =
             a.ranked ? exact_taat_splits(q.n, a.post.n_chunks, a.post.chunk_docs, sms) : 1;
         const size_t cands = static_cast<size_t>(q.n) * a.post.n_chunks * a.splits * k;

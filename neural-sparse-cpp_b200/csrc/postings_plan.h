@@ -35,7 +35,7 @@ NSP_POSTINGS_HD inline void each_posting(int32_t lo, int32_t hi, int64_t first, 
 }
 
 // Whether no score can leave the finite numbers: a bound on every partial sum
-// of products from the largest magnitude stored and the largest sum of a
+// of products from the largest magnitude stored and a bound on the sum of a
 // query's magnitudes (65,536 roundings add less than half a percent). Not so
 // where either is infinite or NaN.
 inline bool finite_scores(float max_abs, double query_abs) {
