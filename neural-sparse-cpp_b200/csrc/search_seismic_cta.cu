@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(1024, 1) seismic_cta_kernel(SeismicLaunch a) {
                         else
                             score_batch<V, TE, false, kG>(a.fwd, ctl, tbl, qv, coff, clen,
                                                           csc, total, lane);
-                                        __syncthreads();
+                        __syncthreads();
                     }
                     // 7. second pruning test and heap offers, in block order.
                     // (a) All threads: a doc can still enter the heap only if
