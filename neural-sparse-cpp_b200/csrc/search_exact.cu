@@ -510,7 +510,12 @@ __global__ void __launch_bounds__(kTThreads) exact_taat_kernel(ExactLaunch a) {
     float* tqv = reinterpret_cast<float*>(thi + kTermWin);
     float* lsd = tqv + kTermWin;
     int32_t* lsi = reinterpret_cast<int32_t*>(lsd + kTWarps * a.k);
-    __shared__ SelectShared sh;
+    // The select's words take the query values' place, which are done with by
+    // then: the dynamic size above is a quarter of the SM's shared memory to the
+    // byte, and 48 bytes of static memory beside it left three CTAs per SM
+    // resident instead of four.
+    SelectShared& sh = *reinterpret_cast<SelectShared*>(tqv);
+    static_assert(sizeof(SelectShared) <= kTermWin * sizeof(float), "the select's words fit");
 
     const int32_t d0 = c * P.chunk_docs + part * part_docs;
     const int nd = max(0, min(part_docs, a.fwd.n_docs - d0));
