@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(32) exact_merge_kernel(const float* cand_d, co
 //
 // A chunk may be split over several CTAs (`splits`), each taking an equal
 // part of its docs: a few queries would otherwise leave most of the GPU idle
-// (7 queries on 300,000 docs: 189 CTAs of 11,264 docs). A CTA finds its part
+// (7 queries on 300,000 docs: 189 CTAs of 11,520 docs). A CTA finds its part
 // of each term's run by binary search over the run's doc ids.
 //
 // The chunk's top k: a radix select over order-preserving score keys (11, 11
@@ -330,10 +330,12 @@ __global__ void __launch_bounds__(32) exact_merge_kernel(const float* cand_d, co
 // Terms of a large share of the docs are applied from dense rows (postings.cu)
 // with vector loads and, over a run of such terms, the scores in registers.
 //
-// Measured (whole calls): 1,000 queries, k = 10, on 100,000 docs 1.73 -> 1.03
-// ms, bound by the L1 data pipe before (a read-modify-write per posting) and
-// by L2 reads of the dense rows now; 7 filtered queries, k = 100, on 300,001
-// docs 579 -> 209 us, bound by each CTA's chain of terms.
+// Measured (whole calls): 1,000 queries, k = 10, on 100,000 docs 1.73 -> 0.89
+// ms, bound by the L1 data pipe before (a read-modify-write per posting); now
+// by instruction issue (67% of the slots) and the L1 data pipe (61%) with four
+// CTAs of 8 warps per SM: the dense rows' L2 reads, 5.7 GB in 0.82 ms, are 20%
+// of that path's rate. 7 filtered queries, k = 100, on 300,001 docs 579 -> 171
+// us, bound by each CTA's chain of terms.
 constexpr int kTWarps = 8;
 constexpr int kTThreads = kTWarps * 32;
 constexpr int kTermWin = 256;  // query terms whose runs are located at once

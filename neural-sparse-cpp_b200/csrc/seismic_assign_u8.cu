@@ -19,8 +19,7 @@
 //              stream through two 32 KB stages of 128 terms x <= 256
 //              centroids (cp.async, 128-byte swizzle), one thread issues the
 //              MMAs, and the warps move the accumulators to the CTA's scratch
-//              rows in global memory (at most 0.5 MB per CTA, so they stay in
-//              L2);
+//              rows in global memory (at most 0.5 MB per CTA, mostly in L2);
 //   then       a warp per doc adds the sparse products from the list's
 //              term-major index of the centroids' other terms (shared-memory
 //              integer atomics; a bitmap of the indexed terms spares the
@@ -33,9 +32,12 @@
 // Measured (SEISMIC-SQ, 200,000 docs, lambda 6000, beta 600: 7.9M docs to
 // assign in 5,175 lists): the assignment phase 370 -> 80 ms, this kernel 45 ms
 // of it. Per tile of 128 docs, in thousands of cycles: centroid stages and
-// MMAs 58 (two stages in flight: bound by the L2 round trips of the centroid
-// rows, not by the tensor cores), accumulators to scratch 17, sparse products
-// and argmax 99 (issue and L2 latency); 290 per list for its index.
+// MMAs 58 (two stages in flight: bound by the round trips of the centroid
+// rows, not by the tensor cores, whose pipe is active 5% of the time),
+// accumulators to scratch 17, sparse products and argmax 99 (issue and L2
+// latency); 290 per list for its index. No pipe is near its peak (100,000
+// docs: issue 49%, L1 data pipe 36%, DRAM 1.9 TB/s, L2 hits 49%): waits for
+// memory and barriers are most of the stalls.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -573,8 +575,12 @@ bool assign_u8(const FwdView& f, const AssignLists& lists, const std::vector<int
     const int n_hot = std::min(dim, hot_bytes);
     std::partial_sort(by_df.begin(), by_df.begin() + n_hot, by_df.end(),
                       [&](int32_t x, int32_t y) { return df[x] != df[y] ? df[x] > df[y] : x < y; });
-    // the share of a random pair's products on hot terms: below half, the
-    // dense part is not worth its multiply-adds
+    // The share of a random pair's products on hot terms: from half on the
+    // dense part is worth its multiply-adds. The assignment phase here against
+    // the general kernel (100,000 docs, lambda 3000, beta 300, terms Zipf(s)):
+    // s = 1.1, share 0.99: 18 against 115 ms; 0.5, 0.65: 39 against 143; 0.3,
+    // 0.24: 50 against 178, so the line is on the safe side, and corpora below
+    // it, whose terms are close to evenly spread, were not measured further.
     double hot_sq = 0.0, all_sq = 0.0;
     for (int i = 0; i < dim; ++i) {
         const double x = static_cast<double>(df[by_df[i]]);

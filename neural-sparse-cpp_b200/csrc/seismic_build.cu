@@ -322,7 +322,10 @@ __global__ void __launch_bounds__(1024) assign_kernel(AssignArgs a) {
     // that at least 40% of the list's centroids hold is therefore applied as a
     // dense row of shared memory, four centroids per lane and no conflicts
     // (below that share the row's zero products cost more than the conflicts:
-    // with 20% the case below takes 84 ms, with 30% 80);
+    // with 20% the case below takes 84 ms, with 30% 80. With 30 / 40 / 60%:
+    // docs of median 120 terms, 80,000 of them, lambda 4000, beta 400 97 / 93 /
+    // 96 ms; 60,000, 6000, 750 101 / 94 / 92; 40,000, 1000, 100 and 20,000,
+    // 2500, 125 the same 37 and 25 with all three);
     // centroids without the term add a zero product, which leaves a sum as it
     // is while the doc's value is finite. Staging the other terms' runs in
     // shared memory as well, 32 terms at a time, was slower: the stage is more
